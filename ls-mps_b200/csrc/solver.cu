@@ -1,10 +1,7 @@
 // PPE solvers on sm_100a.
 //
 // * REFERENCE: the reference's unpreconditioned FP64 BiCGStab (src/lsmps.cpp:65-67)
-//   reproduced bit for bit: exactly rounded FP64 vector updates in the reference's
-//   expression order, row-sequential SpMV in stored entry order, and dot products summed
-//   sequentially in the reference's unknown order by one thread (products formed in
-//   parallel). Slow by design; it exists so small cases match the reference exactly.
+//   reproduced bit for bit (exact.cu).
 // * FP64 / JACOBI: the same iteration with GPU reductions. Jacobi right preconditioning
 //   is applied as a column scaling of the matrix (A D^-1, solve for y, x = D^-1 y), which
 //   costs nothing per iteration.
@@ -38,134 +35,6 @@ namespace {
 
 constexpr int RB = 256;            // threads per block
 constexpr int RGRID = 148 * 6;     // persistent grid of the vector / SpMV kernels
-
-// ---------------------------------------------------------------------------------------
-// REFERENCE (bit-exact) solver
-// ---------------------------------------------------------------------------------------
-struct ExactState {
-    double rho, rho0, alpha, omega, beta, bnorm, thresh, den, tt;
-    int done;    // 1 converged, 2 break
-    int s_conv;
-    int iters;
-    int it;
-    int converged;
-};
-
-__global__ void k_x_prod(const double* __restrict__ a, const double* __restrict__ b,
-                         const int* __restrict__ u_of_ref, long long U, double* __restrict__ prod,
-                         const ExactState* st) {
-    if (st->done) return;
-    for (long long rr = blockIdx.x * (long long)blockDim.x + threadIdx.x; rr < U;
-         rr += (long long)gridDim.x * blockDim.x) {
-        int u = u_of_ref[rr];
-        prod[rr] = xmul(a[u], b[u]);
-    }
-}
-
-enum ExactOp { OP_BNORM, OP_RHO, OP_DEN, OP_SN, OP_TT, OP_TS, OP_RN };
-
-// One thread: sequential sum (the reference's dot, src/lsmps.cpp:66) and the scalar step.
-__global__ void k_x_tail(const double* __restrict__ prod, long long U, ExactState* st, int op, double tol,
-                         int max_iter) {
-    if (threadIdx.x || blockIdx.x) return;
-    if (st->done) return;
-    double s = 0;
-    for (long long rr = 0; rr < U; ++rr) s = xadd(s, prod[rr]);
-    switch (op) {
-        case OP_BNORM:
-            st->bnorm = __dsqrt_rn(s);
-            st->thresh = xmul(tol, fmax(1.0, st->bnorm));
-            st->rho0 = st->alpha = st->omega = 1.0;
-            st->it = 0;
-            st->iters = 0;
-            if (max_iter <= 0) st->done = 2;
-            break;
-        case OP_RHO:
-            st->rho = s;
-            if (fabs(s) < 1e-30) { st->done = 2; break; }
-            st->beta = xmul(xdiv(st->rho, st->rho0), xdiv(st->alpha, st->omega));
-            break;
-        case OP_DEN:
-            if (fabs(s) < 1e-30) { st->done = 2; break; }
-            st->alpha = xdiv(st->rho, s);
-            break;
-        case OP_SN:
-            if (__dsqrt_rn(s) <= st->thresh) { st->s_conv = 1; st->iters = st->it + 1; st->converged = 1; }
-            break;
-        case OP_TT:
-            st->tt = s;
-            if (s < 1e-30) st->done = 2;
-            break;
-        case OP_TS:
-            st->omega = xdiv(s, st->tt);
-            break;
-        case OP_RN:
-            st->iters = st->it + 1;
-            if (__dsqrt_rn(s) <= st->thresh) { st->converged = 1; st->done = 1; break; }
-            if (fabs(st->omega) < 1e-30) { st->done = 2; break; }
-            st->rho0 = st->rho;
-            st->it += 1;
-            if (st->it >= max_iter) st->done = 2;
-            break;
-    }
-}
-
-__global__ void k_x_spmv(long long U, const int* __restrict__ row, const int* __restrict__ col,
-                         const double* __restrict__ val, const double* __restrict__ x, double* __restrict__ y,
-                         const ExactState* st, int check) {
-    if (check && st->done) return;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < U;
-         i += (long long)gridDim.x * blockDim.x) {
-        double s = 0;
-        for (int e = row[i]; e < row[i + 1]; ++e) s = xadd(s, xmul(val[e], x[col[e]]));
-        y[i] = s;
-    }
-}
-
-// kind 0: p = r + beta (p - omega v); 1: s = r - alpha v; 2: x += alpha p (and finish when
-// the |s| test passed); 3: x += alpha p + omega s, r = s - omega t.
-__global__ void k_x_vec(long long U, int kind, double* __restrict__ x, double* __restrict__ r,
-                        double* __restrict__ p, const double* __restrict__ v, double* __restrict__ s,
-                        const double* __restrict__ t, ExactState* st) {
-    if (st->done) return;
-    if (kind == 2 && !st->s_conv) return;
-    if (kind == 3 && st->s_conv) return;
-    const double alpha = st->alpha, beta = st->beta, omega = st->omega;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < U;
-         i += (long long)gridDim.x * blockDim.x) {
-        if (kind == 0) p[i] = xadd(r[i], xmul(beta, xsub(p[i], xmul(omega, v[i]))));
-        else if (kind == 1) s[i] = xsub(r[i], xmul(alpha, v[i]));
-        else if (kind == 2) { x[i] = xadd(x[i], xmul(alpha, p[i])); r[i] = s[i]; }
-        else {
-            x[i] = xadd(x[i], xadd(xmul(alpha, p[i]), xmul(omega, s[i])));
-            r[i] = xsub(s[i], xmul(omega, t[i]));
-        }
-    }
-}
-
-__global__ void k_x_finish_sconv(ExactState* st) {
-    if (st->s_conv && !st->done) st->done = 1;
-}
-
-// Final statistics (src/lsmps.cpp:67 tail): sequential sums in reference order.
-__global__ void k_x_final(const double* __restrict__ Ax, const double* __restrict__ b,
-                          const double* __restrict__ x, const double* __restrict__ xe,
-                          const int* __restrict__ u_of_ref, long long U, double* out) {
-    if (threadIdx.x || blockIdx.x) return;
-    double res = 0, se = 0, mx = 0, exn = 0;
-    for (long long rr = 0; rr < U; ++rr) {
-        int u = u_of_ref[rr];
-        double d = xsub(Ax[u], b[u]);
-        res = xadd(res, xmul(d, d));
-        double e = xsub(x[u], xe[u]);
-        se = xadd(se, xmul(e, e));
-        exn = xadd(exn, xmul(xe[u], xe[u]));
-        mx = fmax(mx, fabs(e));
-    }
-    out[0] = __dsqrt_rn(res);
-    out[1] = __dsqrt_rn(xdiv(se, fmax(exn, 1e-30)));
-    out[2] = mx;
-}
 
 // ---------------------------------------------------------------------------------------
 // Fast engine
@@ -1431,87 +1300,6 @@ void set_scalar_caps(Engine& E, int max_iter, int stall_window) {
 }  // namespace
 
 // ---------------------------------------------------------------------------------------
-static void solve_exact(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_stats* ps) {
-    cudaStream_t s = ctx->stream;
-    long long U = ctx->U;
-    double* x = ctx->vx.ensure<double>(U + 1);
-    double* r = ctx->vr.ensure<double>(U + 1);
-    double* r0 = ctx->vr0.ensure<double>(U + 1);
-    double* p = ctx->vp.ensure<double>(U + 1);
-    double* v = ctx->vv.ensure<double>(U + 1);
-    double* sv = ctx->vs.ensure<double>(U + 1);
-    double* t = ctx->vt.ensure<double>(U + 1);
-    double* prod = ctx->vph.ensure<double>(U + 1);
-    ExactState* st = reinterpret_cast<ExactState*>(ctx->red.ensure<double>(64));
-    const double* b = ctx->A_b.get<double>();
-    const int* uref = ctx->u_of_ref.get<int>();
-    const int* row = ctx->A_row.get<int>();
-    const int* col = ctx->A_col.get<int>();
-    const double* val = ctx->A_val.get<double>();
-    LSMPS_CUDA(cudaMemsetAsync(st, 0, sizeof(ExactState), s));
-    LSMPS_CUDA(cudaMemsetAsync(x, 0, U * sizeof(double), s));
-    LSMPS_CUDA(cudaMemsetAsync(p, 0, U * sizeof(double), s));
-    LSMPS_CUDA(cudaMemsetAsync(v, 0, U * sizeof(double), s));
-    LSMPS_CUDA(cudaMemcpyAsync(r, b, U * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    LSMPS_CUDA(cudaMemcpyAsync(r0, b, U * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    const unsigned G = 148 * 4, B = 256;
-    const int max_iter = o->max_iter;
-    const double tol = o->tol;
-    auto dot = [&](const double* a, const double* c, int op) {
-        k_x_prod<<<G, B, 0, s>>>(a, c, uref, U, prod, st);
-        k_x_tail<<<1, 32, 0, s>>>(prod, U, st, op, tol, max_iter);
-    };
-    ev_record(ctx, 10);
-    if (U > 0) {
-        dot(b, b, OP_BNORM);
-        const int check = std::max(1, o->check_every > 0 ? o->check_every : 16);
-        for (int it = 0; it < max_iter; ++it) {
-            dot(r0, r, OP_RHO);
-            k_x_vec<<<G, B, 0, s>>>(U, 0, x, r, p, v, sv, t, st);
-            k_x_spmv<<<G, B, 0, s>>>(U, row, col, val, p, v, st, 1);
-            dot(r0, v, OP_DEN);
-            k_x_vec<<<G, B, 0, s>>>(U, 1, x, r, p, v, sv, t, st);
-            dot(sv, sv, OP_SN);
-            k_x_vec<<<G, B, 0, s>>>(U, 2, x, r, p, v, sv, t, st);
-            k_x_finish_sconv<<<1, 1, 0, s>>>(st);
-            k_x_spmv<<<G, B, 0, s>>>(U, row, col, val, sv, t, st, 1);
-            dot(t, t, OP_TT);
-            dot(t, sv, OP_TS);
-            k_x_vec<<<G, B, 0, s>>>(U, 3, x, r, p, v, sv, t, st);
-            dot(r, r, OP_RN);
-            LSMPS_CHECK_LAUNCH();
-            note_launches(18);
-            if ((it + 1) % check == 0) {
-                int done = 0;
-                LSMPS_CUDA(cudaMemcpyAsync(&done, &st->done, sizeof(int), cudaMemcpyDeviceToHost, s));
-                LSMPS_CUDA(cudaStreamSynchronize(s));
-                if (done) break;
-            }
-        }
-    }
-    ev_record(ctx, 11);
-    ExactState h{};
-    LSMPS_CUDA(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    double fin[3] = {0, 0, 0};
-    if (U > 0) {
-        k_x_spmv<<<G, B, 0, s>>>(U, row, col, val, x, t, st, 0);
-        double* out = reinterpret_cast<double*>(st + 1);
-        k_x_final<<<1, 32, 0, s>>>(t, b, x, ctx->A_xexact.get<double>(), uref, U, out);
-        LSMPS_CHECK_LAUNCH();
-        LSMPS_CUDA(cudaMemcpyAsync(fin, out, sizeof(fin), cudaMemcpyDeviceToHost, s));
-    }
-    LSMPS_CUDA(cudaStreamSynchronize(s));
-    ps->iterations = h.iters;
-    ps->converged = h.converged;
-    ps->initial_residual = h.bnorm;
-    ps->final_residual = fin[0];
-    ps->relative_l2_error = fin[1];
-    ps->max_error = fin[2];
-    ps->relative_residual = fin[0] / std::max(h.bnorm, 1e-300);
-    ps->solve_ms = ev_elapsed(ctx, 10, 11);
-}
-
-
 // ---- SELL-32 copies of the assembled matrix (built on first use after an assembly) ----
 static void sell_raw(lsmps_ctx* ctx);
 // kind 0: A (FP64), 1: A D^-1 (FP64), 2: A D^-1 (FP32)

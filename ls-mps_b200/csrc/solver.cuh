@@ -57,4 +57,7 @@ struct MgFine {
 };
 MgFine mg_fine(lsmps_ctx* ctx);
 
+// exact.cu: the REFERENCE solver (bit-identical to the reference's BiCGStab)
+void solve_exact(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_stats* ps);
+
 }  // namespace lsmps_gpu
