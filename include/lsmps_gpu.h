@@ -95,8 +95,8 @@ int lsmps_kernel_bench(lsmps_ctx* ctx, int kernel, int reps, double* ms_per_laun
 /* Launch-shape autotuner. Kernels whose launch shapes (grid size, block size, loads in
  * flight) all give the same bits time each shape once on the live data at their first use
  * per problem-size class (floor(log2 n)) and keep the fastest for the context: the network's
- * message-passing layer and the all-particle WLS. mode 0: off (fixed default shapes), 1: on
- * (default), 2: on and forget earlier choices. No reference counterpart. */
+ * message-passing layer. mode 0: off (fixed default shape), 1: on (default), 2: on and forget
+ * earlier choices. No reference counterpart. */
 int lsmps_set_autotune(lsmps_ctx* ctx, int mode);
 /* The tuner's table as text, one line per candidate: "kernel n~2^k<TAB>shape<TAB>ms[<TAB>best]".
  * Writes at most cap bytes (NUL-terminated) to buf; *needed gets the full size + 1. */

@@ -217,7 +217,7 @@ void lsmps_ctx_destroy(lsmps_ctx* ctx) {
                                  &ctx->scell, &ctx->cls, &ctx->nbr_cnt, &ctx->nbr_row, &ctx->nbr_col, &ctx->seg_list,
                                  &ctx->cand_row, &ctx->cand_col, &ctx->ref_sx, &ctx->ref_sy, &ctx->ref_sz,
                                  &ctx->nbr_stats, &ctx->wls_status, &ctx->wls_z, &ctx->wls_wsum, &ctx->wls_x,
-                                 &ctx->wf_in, &ctx->wf_x, &ctx->wf_status, &ctx->wf_z, &ctx->wf_wsum, &ctx->wf_stats,
+                                 &ctx->wf_in, &ctx->wf_status, &ctx->wf_z, &ctx->wf_wsum, &ctx->wf_stats,
                                  &ctx->pj_grad, &ctx->pj_gradp, &ctx->pj_div, &ctx->pj_mask, &ctx->pj_stats,
                                  &ctx->pj_hop, &ctx->ld_ident, &ctx->S_dcol, &ctx->S_rbase,
                                  &ctx->wls_stats, &ctx->wls_sample, &ctx->wls_sq, &ctx->ref_rank, &ctx->u_of_sorted,

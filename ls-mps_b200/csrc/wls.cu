@@ -14,8 +14,9 @@
 // PPE rows use. Precision 1 factors in FP32 and refines each solve against the FP64 M;
 // a system whose FP32 factorisation fails or that needed regularisation is refactored
 // in FP64.
+#include <algorithm>
 #include <cmath>
-#include <vector>
+#include <cstring>
 
 #include "ops.cuh"
 #include "seqsum.cuh"
@@ -259,9 +260,11 @@ struct WlsParams {
     double coef[30];  // nrhs x 10
 };
 
-__device__ __forceinline__ double quad_fast(const double* c, double x, double y, double z) {
-    return c[0] + c[1] * x + c[2] * y + c[3] * z + c[4] * x * x + c[5] * y * y + c[6] * z * z + c[7] * x * y +
-           c[8] * x * z + c[9] * y * z;
+// gradient of the quadratic field c at (x, y, z)
+__device__ __forceinline__ void quad_grad(const double* c, double x, double y, double z, double* g) {
+    g[0] = c[1] + 2 * c[4] * x + c[7] * y + c[8] * z;
+    g[1] = c[2] + 2 * c[5] * y + c[7] * x + c[9] * z;
+    g[2] = c[3] + 2 * c[6] * z + c[8] * x + c[9] * y;
 }
 
 // Every basis function of the reference (src/lsmps.cpp:23) is one power of 1/r times a monomial
@@ -353,7 +356,7 @@ __device__ __forceinline__ double accumulate_moments_rhs(int k, const double* __
                                                          const int* __restrict__ row, const int* __restrict__ col,
                                                          const uint8_t* __restrict__ cls, const WlsParams& P,
                                                          double l0inv, const double* __restrict__ fvals,
-                                                         const double* fi, double* M, double (*B)[K]) {
+                                                         double* M, double (*B)[K]) {
     double T[NMONO];
 #pragma unroll
     for (int t = 0; t < NMONO; ++t) T[t] = 0;
@@ -363,10 +366,25 @@ __device__ __forceinline__ double accumulate_moments_rhs(int k, const double* __
         for (int a = 0; a < K; ++a) B[f][a] = 0;
     const double xi = sx[k], yi = sy[k], zi = sz[k];
     double ws = 0;
-    for (int e = row[k]; e < row[k + 1]; ++e) {
-        const int m = col[e];
-        const double xm = sx[m], ym = sy[m], zm = sz[m];
-        const double dx = xm - xi, dy = ym - yi, dz = zm - zi;
+    double fi[NRHS], gf[NRHS][3];  // the field's value at k (array), or its gradient there
+#pragma unroll
+    for (int f = 0; f < NRHS; ++f) {
+        fi[f] = fvals ? fvals[(size_t)k * NRHS + f] : 0.0;
+        quad_grad(P.coef + 10 * f, xi, yi, zi, gf[f]);
+    }
+    // the next neighbor's position (and the index after it) are loaded while this one's terms
+    // are summed
+    const int e1 = row[k + 1];
+    int e = row[k];
+    int m = e < e1 ? col[e] : 0, mn = e + 1 < e1 ? col[e + 1] : 0;
+    double xm = sx[m], ym = sy[m], zm = sz[m];
+    for (; e < e1; ++e) {
+        const int mc = m;
+        const double xc = xm, yc = ym, zc = zm;
+        m = mn;
+        xm = sx[m], ym = sy[m], zm = sz[m];
+        mn = e + 2 < e1 ? col[e + 2] : 0;
+        const double dx = xc - xi, dy = yc - yi, dz = zc - zi;
         const double r2 = dx * dx + dy * dy + dz * dz;
         if (!(r2 > 1e-24) || r2 >= P.re * P.re) continue;  // r <= 1e-12 or r >= re: weight 0
         const double ir = rsqrt(r2);                         // 1 / r without a square root and a division
@@ -376,11 +394,15 @@ __device__ __forceinline__ double accumulate_moments_rhs(int k, const double* __
         const double p[6] = {dx * dx, dx * dy, dx * dz, dy * dy, dy * dz, dz * dz};
         ws += w;
         add_monomials(W, dx, dy, dz, p, T);
-        if (P.mirror_walls && cls[m] == LSMPS_WALL) continue;  // f_m = f_k: no right-hand-side term
+        if (P.mirror_walls && cls[mc] == LSMPS_WALL) continue;  // f_m = f_k: no right-hand-side term
 #pragma unroll
         for (int f = 0; f < NRHS; ++f) {
-            const double fm = fvals ? fvals[(size_t)m * NRHS + f] : quad_fast(P.coef + 10 * f, xm, ym, zm);
-            const double g = (fm - fi[f]) * W;
+            // f_m - f_k; of a quadratic field from its gradient at k and its second derivatives
+            const double* c = P.coef + 10 * f;
+            const double df = fvals ? fvals[(size_t)mc * NRHS + f] - fi[f]
+                                    : gf[f][0] * dx + gf[f][1] * dy + gf[f][2] * dz + c[4] * p[0] + c[5] * p[3] +
+                                          c[6] * p[5] + c[7] * p[1] + c[8] * p[2] + c[9] * p[4];
+            const double g = df * W;
             B[f][0] += g * dx, B[f][1] += g * dy, B[f][2] += g * dz;
             B[f][3] += g * p[0], B[f][4] += g * p[3], B[f][5] += g * p[5];
             B[f][6] += g * p[1], B[f][7] += g * p[2], B[f][8] += g * p[4];
@@ -438,35 +460,40 @@ __device__ __forceinline__ void solve_packed(const T* L, T* x) {  // x holds b o
     }
 }
 
-// Per-block statistics: counts (u64) [0] ok [1] reg [2] skip [3] noweight [4] cholfail
-// [5] virtual [6] fp64 fallback; sums (f64) [0] se_grad [1] se_lap [2] max_grad [3] max_lap
-struct WlsAccum {
-    unsigned long long cnt[8];
-    double se_g, se_l, mx_g, mx_l;
-};
-
+// Statistics, WLS_SLOTS copies of: counts (u64) [0] ok [1] reg [2] skip [3] noweight [4] cholfail
+// [5] virtual [6] fp64 fallback; sums (f64) [8] se_grad [9] se_lap [10] max_grad [11] max_lap
 __device__ void atomic_max_nonneg(double* addr, double v) {
     atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
 }
 
 // The right-hand sides accumulate in the moments' neighbor pass (one pass over the neighbors;
 // measured 22 % faster at 1M particles than a second right-hand-side pass, for 2 more registers).
-// MINB > 1 caps the registers so that MINB blocks of 128 threads fit an SM (the Cholesky's
-// values spill to L1; the neighbor pass stays in registers).
-template <int NRHS, int PREC, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_wls_all(WlsParams P, int n, const uint8_t* __restrict__ cls,
+// Bound by the FP64 pipe's latency at 12 warps per SM. At 1M particles one field takes 313 us
+// (443 before the neighbor loop loaded one neighbor ahead and took an analytic field's
+// differences from its gradient at k), three caller fields 511 us (874, and 386 more for the copy
+// of the solutions to the caller's order, where they are now written directly).
+// One warp per block, so a warp's registers are free for the next one as soon as it ends (rows
+// of uneven length): blocks of 64 and 128 threads took 5 and 17 % longer.
+// Registers: one FP64 field takes 166 by itself, 12 warps per SM. Two and three fields would take
+// 192-216 (8-10 warps) and are capped at 168: 464 against 597 us (two) and 651 against 649
+// (three) at 1M, 32 against 46 and 42 against 50 at 50k. Mixed precision with one field is capped
+// too (499 against 562 us at 1M), with more the spills cost more than the warps gain (three
+// fields at 100k: 139 capped against 113).
+template <int NRHS, int PREC>
+constexpr int wls_regs() {
+    return (NRHS == 1) == (PREC == 0) ? 255 : 168;
+}
+constexpr int WLS_SLOTS = 16;  // copies of the statistics, so that the blocks' atomics spread
+template <int NRHS, int PREC>
+__global__ void __maxnreg__((wls_regs<NRHS, PREC>())) k_wls_all(WlsParams P, int n, const uint8_t* __restrict__ cls,
                                                  const double* __restrict__ sx, const double* __restrict__ sy,
                                                  const double* __restrict__ sz, const int* __restrict__ row,
                                                  const int* __restrict__ col, int* __restrict__ status,
                                                  double* __restrict__ zout, double* __restrict__ wsum,
                                                  double* __restrict__ xout, unsigned long long* gcnt,
-                                                 double* gsum, const double* __restrict__ fvals) {
-    __shared__ unsigned long long s_cnt[8];
-    __shared__ double s_sum[4];
-    if (threadIdx.x < 8) s_cnt[threadIdx.x] = 0;
-    if (threadIdx.x < 4) s_sum[threadIdx.x] = 0;
-    __syncthreads();
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
+                                                 const double* __restrict__ fvals,
+                                                 const int* __restrict__ xperm) {
+    int k = blockIdx.x * 32 + threadIdx.x;
     int my_status = -1, my_virt = 0, my_fb = 0;
     double se_g = 0, se_l = 0, mx_g = 0, mx_l = 0;
     if (k < n) {
@@ -482,13 +509,7 @@ __global__ void __launch_bounds__(128, MINB) k_wls_all(WlsParams P, int n, const
             const double xi = sx[k], yi = sy[k], zi = sz[k];
             // right-hand sides: the quadratic fields (the Laplacian vector is solved separately)
             double B[NRHS][K];
-            // field values: per-particle array (sorted order, NRHS per particle) or the
-            // analytic quadratics
-            double fi[NRHS];
-#pragma unroll
-            for (int f = 0; f < NRHS; ++f)
-                fi[f] = fvals ? fvals[(size_t)k * NRHS + f] : quad_fast(P.coef + 10 * f, xi, yi, zi);
-            double ws = accumulate_moments_rhs<NRHS>(k, sx, sy, sz, row, col, cls, P, l0inv, fvals, fi, L, B);
+            double ws = accumulate_moments_rhs<NRHS>(k, sx, sy, sz, row, col, cls, P, l0inv, fvals, L, B);
             wsum[k] = ws;
             if (!(ws > 0)) {
                 my_status = W_NOWEIGHT;
@@ -586,16 +607,17 @@ __global__ void __launch_bounds__(128, MINB) k_wls_all(WlsParams P, int n, const
                     for (int a = 0; a < K; ++a) zout[(size_t)k * K + a] = z[a];
 #pragma unroll
                     for (int f = 0; f < NRHS; ++f) {
-                        if (P.store)
+                        if (P.store) {
+                            const size_t o = ((size_t)(xperm ? xperm[k] : k) * NRHS + f) * K;
 #pragma unroll
-                            for (int a = 0; a < K; ++a) xout[((size_t)k * NRHS + f) * K + a] = B[f][a];
+                            for (int a = 0; a < K; ++a) xout[o + a] = B[f][a];
+                        }
                         if (fvals) continue;  // no analytic field to measure against
                         const double* c = P.coef + 10 * f;
-                        double gx = c[1] + 2 * c[4] * xi + c[7] * yi + c[8] * zi;
-                        double gy = c[2] + 2 * c[5] * yi + c[7] * xi + c[9] * zi;
-                        double gz = c[3] + 2 * c[6] * zi + c[8] * xi + c[9] * yi;
+                        double gr[3];
+                        quad_grad(c, xi, yi, zi, gr);
                         double lap = 2 * (c[4] + c[5] + c[6]);
-                        double ex = B[f][0] - gx, ey = B[f][1] - gy, ez = B[f][2] - gz;
+                        double ex = B[f][0] - gr[0], ey = B[f][1] - gr[1], ez = B[f][2] - gr[2];
                         double ge = sqrt(ex * ex + ey * ey + ez * ez);
                         double le = fabs((B[f][3] + B[f][4] + B[f][5]) * l0inv - lap);
                         se_g += ge * ge;
@@ -607,11 +629,13 @@ __global__ void __launch_bounds__(128, MINB) k_wls_all(WlsParams P, int n, const
             }
         }
         status[k] = my_status;
+        if (P.store && my_status > W_REG) {  // no solution: zeros
+            const size_t o = (size_t)(xperm ? xperm[k] : k) * NRHS * K;
+#pragma unroll
+            for (int a = 0; a < NRHS * K; ++a) xout[o + a] = 0;
+        }
     }
-    // block reduction of the statistics
-    if (my_status >= 0) atomicAdd(&s_cnt[my_status], 1ull);
-    if (my_virt) atomicAdd(&s_cnt[5], 1ull);
-    if (my_fb) atomicAdd(&s_cnt[6], 1ull);
+    // the warp's statistics
     se_g = warp_sum(se_g);
     se_l = warp_sum(se_l);
 #pragma unroll
@@ -619,63 +643,38 @@ __global__ void __launch_bounds__(128, MINB) k_wls_all(WlsParams P, int n, const
         mx_g = fmax(mx_g, __shfl_xor_sync(0xffffffffu, mx_g, o));
         mx_l = fmax(mx_l, __shfl_xor_sync(0xffffffffu, mx_l, o));
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&s_sum[0], se_g);
-        atomicAdd(&s_sum[1], se_l);
-        atomic_max_nonneg(&s_sum[2], mx_g);
-        atomic_max_nonneg(&s_sum[3], mx_l);
+    unsigned long long* cnt = gcnt + 16 * (blockIdx.x % WLS_SLOTS);
+    double* sum = reinterpret_cast<double*>(cnt + 8);
+#pragma unroll
+    for (int c = 0; c < 7; ++c) {
+        const unsigned m = __ballot_sync(0xffffffffu, c < 5 ? my_status == c : c == 5 ? my_virt : my_fb);
+        if (m && threadIdx.x == c) atomicAdd(&cnt[c], (unsigned long long)__popc(m));
     }
-    __syncthreads();
-    if (threadIdx.x < 7 && s_cnt[threadIdx.x]) atomicAdd(&gcnt[threadIdx.x], s_cnt[threadIdx.x]);
-    if (threadIdx.x == 0) {
-        atomicAdd(&gsum[0], s_sum[0]);
-        atomicAdd(&gsum[1], s_sum[1]);
-        atomic_max_nonneg(&gsum[2], s_sum[2]);
-        atomic_max_nonneg(&gsum[3], s_sum[3]);
-    }
+    if (threadIdx.x == 0 && se_g != 0) atomicAdd(&sum[0], se_g);
+    if (threadIdx.x == 0 && se_l != 0) atomicAdd(&sum[1], se_l);
+    if (threadIdx.x == 0 && mx_g > 0) atomic_max_nonneg(&sum[2], mx_g);
+    if (threadIdx.x == 0 && mx_l > 0) atomic_max_nonneg(&sum[3], mx_l);
 }
 
-// Launch shapes the autotuner chooses from (one particle per thread: same bits for each):
-// blocks of 32, 64 or 128 threads with the compiler's register count, and (single field) 128
-// threads capped at 128 registers for four blocks per SM.
-constexpr int WLS_BLOCK[4] = {32, 64, 128, 128};
-
-// Outputs of one all-particle WLS launch (sorted order).
+// Outputs of one all-particle WLS launch (sorted order; x row k at xperm[k] when that is set).
 struct WlsOut {
     int* status;
     double *z, *wsum, *x;
+    const int* xperm = nullptr;
 };
 
 template <int NRHS, int PREC>
-void launch_all(lsmps_ctx* ctx, const WlsParams& P, unsigned long long* gcnt, double* gsum,
+void launch_all(lsmps_ctx* ctx, const WlsParams& P, unsigned long long* gcnt,
                 const double* fvals = nullptr, const WlsOut* dst = nullptr) {
     int n = (int)ctx->n;
     if (!n) return;
     const WlsOut o = dst ? *dst
                          : WlsOut{ctx->wls_status.get<int>(), ctx->wls_z.get<double>(), ctx->wls_wsum.get<double>(),
                                   ctx->wls_x.get<double>()};
-    constexpr bool capped = NRHS == 1;  // the register-capped shape exists for one field
-    auto go = [&](int c) {
-        const int t = WLS_BLOCK[c];
-        if (capped && c == 3)
-            k_wls_all<NRHS, PREC, capped ? 4 : 1><<<blocks_for(n, t), t, 0, ctx->stream>>>(
-                P, n, ctx->cls.get<uint8_t>(), ctx->sx.get<double>(), ctx->sy.get<double>(), ctx->sz.get<double>(),
-                ctx->nbr_row.get<int>(), ctx->nbr_col.get<int>(), o.status, o.z, o.wsum, o.x, gcnt, gsum, fvals);
-        else
-            k_wls_all<NRHS, PREC, 1><<<blocks_for(n, t), t, 0, ctx->stream>>>(
-                P, n, ctx->cls.get<uint8_t>(), ctx->sx.get<double>(), ctx->sy.get<double>(), ctx->sz.get<double>(),
-                ctx->nbr_row.get<int>(), ctx->nbr_col.get<int>(), o.status, o.z, o.wsum, o.x, gcnt, gsum, fvals);
-        LSMPS_CHECK_LAUNCH();
-    };
-    static const std::vector<std::string> names3 = {"block32", "block64", "block128"};
-    static const std::vector<std::string> names4 = {"block32", "block64", "block128", "block128 regs128"};
-    const std::string key = "wls_all nrhs" + std::to_string(NRHS) + (PREC ? " mixed" : " fp64");
-    const size_t tuned_before = ctx->tuner.table.size();
-    // without tuning: the capped shape for one field (fastest at 1M), else 128 threads
-    const int c = autotune(ctx, key.c_str(), n, capped ? names4 : names3, capped ? 3 : 2, go);
-    if (ctx->tuner.table.size() != tuned_before)  // the timed launches added to the statistics
-        LSMPS_CUDA(cudaMemsetAsync(gcnt, 0, 16 * sizeof(double), ctx->stream));
-    go(c);
+    k_wls_all<NRHS, PREC><<<blocks_for(n, 32), 32, 0, ctx->stream>>>(
+        P, n, ctx->cls.get<uint8_t>(), ctx->sx.get<double>(), ctx->sy.get<double>(), ctx->sz.get<double>(),
+        ctx->nbr_row.get<int>(), ctx->nbr_col.get<int>(), o.status, o.z, o.wsum, o.x, gcnt, fvals, o.xperm);
+    LSMPS_CHECK_LAUNCH();
 }
 
 // Back to caller order (wls arrays are kept in sorted order).
@@ -748,26 +747,35 @@ void wls_run(lsmps_ctx* ctx, const lsmps_wls_opts* o, lsmps_wls_stats* out) {
     ctx->wls_z.ensure<double>(n * K + 1);
     ctx->wls_wsum.ensure<double>(n + 1);
     ctx->wls_x.ensure<double>(P.store ? n * o->nrhs * K + 1 : 1);
-    auto* gcnt = reinterpret_cast<unsigned long long*>(ctx->wls_stats.ensure<double>(16));
-    double* gsum = reinterpret_cast<double*>(gcnt + 8);
-    LSMPS_CUDA(cudaMemsetAsync(gcnt, 0, 16 * sizeof(double), s));
+    auto* gcnt = reinterpret_cast<unsigned long long*>(ctx->wls_stats.ensure<double>(16 * WLS_SLOTS));
+    LSMPS_CUDA(cudaMemsetAsync(gcnt, 0, 16 * WLS_SLOTS * sizeof(double), s));
     if (P.precision == 0) {
-        if (P.nrhs == 1) launch_all<1, 0>(ctx, P, gcnt, gsum);
-        else if (P.nrhs == 2) launch_all<2, 0>(ctx, P, gcnt, gsum);
-        else launch_all<3, 0>(ctx, P, gcnt, gsum);
+        if (P.nrhs == 1) launch_all<1, 0>(ctx, P, gcnt);
+        else if (P.nrhs == 2) launch_all<2, 0>(ctx, P, gcnt);
+        else launch_all<3, 0>(ctx, P, gcnt);
     } else {
-        if (P.nrhs == 1) launch_all<1, 1>(ctx, P, gcnt, gsum);
-        else if (P.nrhs == 2) launch_all<2, 1>(ctx, P, gcnt, gsum);
-        else launch_all<3, 1>(ctx, P, gcnt, gsum);
+        if (P.nrhs == 1) launch_all<1, 1>(ctx, P, gcnt);
+        else if (P.nrhs == 2) launch_all<2, 1>(ctx, P, gcnt);
+        else launch_all<3, 1>(ctx, P, gcnt);
     }
     ctx->have_wls = true;
     ctx->wls_nrhs = o->nrhs;
     ctx->wls_stored = P.store != 0;
     ctx->have_ppe = ctx->have_solution = false;
     if (!out) return;  // no statistics wanted: no read-back, the host does not wait
-    unsigned long long hc[8];
-    double hs[4];
-    read_back(ctx, {{gcnt, hc, sizeof(hc)}, {gsum, hs, sizeof(hs)}}, nullptr);
+    double slots[WLS_SLOTS][16];
+    read_back(ctx, {{gcnt, slots, sizeof(slots)}}, nullptr);
+    unsigned long long hc[8] = {};
+    double hs[4] = {};
+    for (auto& sl : slots) {
+        for (int c = 0; c < 8; ++c) {
+            unsigned long long v;
+            std::memcpy(&v, &sl[c], sizeof(v));
+            hc[c] += v;
+        }
+        for (int c = 0; c < 2; ++c) hs[c] += sl[8 + c];
+        for (int c = 2; c < 4; ++c) hs[c] = std::max(hs[c], sl[8 + c]);
+    }
     st.ok = hc[W_OK];
     st.regularized = hc[W_REG];
     st.skipped = hc[W_SKIP];
@@ -784,19 +792,12 @@ void wls_run(lsmps_ctx* ctx, const lsmps_wls_opts* o, lsmps_wls_stats* out) {
 }
 
 namespace {
-// caller order (n x nrhs) -> sorted order, and the solutions back
+// caller order (n x nrhs) -> sorted order
 __global__ void k_fields_to_sorted(const int* __restrict__ perm, size_t n, int nrhs, const double* __restrict__ in,
                                    double* __restrict__ out) {
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
         const size_t i = (size_t)perm[k];
         for (int f = 0; f < nrhs; ++f) out[k * nrhs + f] = in[i * nrhs + f];
-    }
-}
-__global__ void k_solutions_to_caller(const int* __restrict__ iperm, size_t n, int nrhs, const double* __restrict__ x,
-                                      double* __restrict__ out) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t k = (size_t)iperm[i];
-        for (int a = 0; a < nrhs * K; ++a) out[i * nrhs * K + a] = x[k * nrhs * K + a];
     }
 }
 }  // namespace
@@ -818,24 +819,17 @@ void wls_fields(lsmps_ctx* ctx, const double* d_fields, int nrhs, double* d_out,
     P.mirror_walls = mirror_walls ? 1 : 0;
     double* fs = ctx->wf_in.ensure<double>(n * nrhs + 1);
     WlsOut o{ctx->wf_status.ensure<int>(n + 1), ctx->wf_z.ensure<double>(n * K + 1), ctx->wf_wsum.ensure<double>(n + 1),
-             ctx->wf_x.ensure<double>(n * nrhs * K + 1)};
-    auto* gcnt = reinterpret_cast<unsigned long long*>(ctx->wf_stats.ensure<double>(16));
-    double* gsum = reinterpret_cast<double*>(gcnt + 8);
-    LSMPS_CUDA(cudaMemsetAsync(gcnt, 0, 16 * sizeof(double), s));
+             d_out, ctx->perm.get<int>()};  // the solutions straight to the caller's order
+    auto* gcnt = reinterpret_cast<unsigned long long*>(ctx->wf_stats.ensure<double>(16 * WLS_SLOTS));
+    LSMPS_CUDA(cudaMemsetAsync(gcnt, 0, 16 * WLS_SLOTS * sizeof(double), s));
     if (n) {
-        LSMPS_CUDA(cudaMemsetAsync(o.x, 0, n * nrhs * K * sizeof(double), s));  // failed rows stay 0
         k_fields_to_sorted<<<std::min<unsigned>(blocks_for(n, 256), 1184), 256, 0, s>>>(ctx->perm.get<int>(), n, nrhs,
                                                                                       d_fields, fs);
         LSMPS_CHECK_LAUNCH();
     }
-    if (nrhs == 1) launch_all<1, 0>(ctx, P, gcnt, gsum, fs, &o);
-    else if (nrhs == 2) launch_all<2, 0>(ctx, P, gcnt, gsum, fs, &o);
-    else launch_all<3, 0>(ctx, P, gcnt, gsum, fs, &o);
-    if (n) {
-        k_solutions_to_caller<<<std::min<unsigned>(blocks_for(n, 256), 1184), 256, 0, s>>>(ctx->iperm.get<int>(), n,
-                                                                                         nrhs, o.x, d_out);
-        LSMPS_CHECK_LAUNCH();
-    }
+    if (nrhs == 1) launch_all<1, 0>(ctx, P, gcnt, fs, &o);
+    else if (nrhs == 2) launch_all<2, 0>(ctx, P, gcnt, fs, &o);
+    else launch_all<3, 0>(ctx, P, gcnt, fs, &o);
 }
 
 void wls_kernel_bench(lsmps_ctx* ctx, int reps, double* ms, double* bytes) {
@@ -847,12 +841,11 @@ void wls_kernel_bench(lsmps_ctx* ctx, int reps, double* ms, double* bytes) {
     P.nrhs = 1;
     const double q[10] = {1, 2, -3, 0.5, 0.7, -0.2, 0.4, 0.3, -0.1, 0.25};
     for (int a = 0; a < 10; ++a) P.coef[a] = q[a];
-    auto* gcnt = reinterpret_cast<unsigned long long*>(ctx->wls_stats.ensure<double>(16));
-    double* gsum = reinterpret_cast<double*>(gcnt + 8);
+    auto* gcnt = reinterpret_cast<unsigned long long*>(ctx->wls_stats.ensure<double>(16 * WLS_SLOTS));
     ctx->wls_x.ensure<double>(1);
-    launch_all<1, 0>(ctx, P, gcnt, gsum);
+    launch_all<1, 0>(ctx, P, gcnt);
     ev_record(ctx, 14);
-    for (int r = 0; r < reps; ++r) launch_all<1, 0>(ctx, P, gcnt, gsum);
+    for (int r = 0; r < reps; ++r) launch_all<1, 0>(ctx, P, gcnt);
     ev_record(ctx, 15);
     *ms = ev_elapsed(ctx, 14, 15) / reps;
     double N = (double)ctx->n, Pp = (double)ctx->pairs;
