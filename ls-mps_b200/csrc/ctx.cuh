@@ -126,7 +126,7 @@ struct lsmps_ctx {
     lsmps_gpu::DevBuf S_ptr, S_len, S_col, S_val, S_vals, S_valf;
     // 16-bit column steps of the SELL copies (used when every row ascends in steps < 65536)
     bool have_steps = false, sell_steps_enabled = true;
-    lsmps_gpu::DevBuf S_dcol, S_rbase;
+    lsmps_gpu::DevBuf S_dcol, S_rbase, S_cut;
 
     // ---- solver state ----
     bool have_solution = false;

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(256) k_x_final(ExactSystem A, const double* __
 void solve_exact(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_stats* ps) {
     cudaStream_t s = ctx->stream;
     const long long U = ctx->U;
-    double* x = ctx->vx.ensure<double>(U + 1);
+    double* x = ctx->vx.ensure<double>(U + 2);
     double* r = ctx->vr.ensure<double>(U + 1);
     double* r0 = ctx->vr0.ensure<double>(U + 1);
     double* p[2] = {ctx->vp.ensure<double>(U + 1), ctx->vs.ensure<double>(U + 1)};

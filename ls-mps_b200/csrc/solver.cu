@@ -5,28 +5,24 @@
 // * FP64 / JACOBI: the same iteration with GPU reductions. Jacobi right preconditioning
 //   is applied as a column scaling of the matrix (A D^-1, solve for y, x = D^-1 y), which
 //   costs nothing per iteration.
-// * MIXED / LEARNED: FP64 iterative refinement, r = b - A x with the FP64 matrix, around
-//   FP32 Jacobi-BiCGStab inner solves of A D^-1 y = r / |r| on an FP32 copy of the matrix.
-//   LEARNED starts each inner solve from the message-passing network's guess.
-//
-// The fast engine runs five kernels per iteration. Each reduction is fused into the
-// kernel that produces its operands; the last block of the grid to finish (atomic ticket)
-// sums the per-block partials in a fixed order, so results are deterministic, and updates
-// the scalars in device memory. Every kernel returns at once when the run is done, so a
-// CUDA graph of several iterations can be replayed without host round trips; the host
-// reads the status once per graph launch.
+// * MIXED / LEARNED: the Jacobi iteration with an FP32 copy of the matrix and residual
+//   replacement by the FP64 one; LEARNED starts from the message-passing network's guess.
+// These run in one cooperative launch per solve (krylov.cu). Here are the SELL copies, the
+// multigrid-preconditioned MIXED / LEARNED iteration and MIXED_F32, whose kernels the host
+// launches: each reduction is fused into the kernel that produces its operands; the last block
+// of the grid to finish (atomic ticket) sums the per-block partials in a fixed order, so results
+// are deterministic, and updates the scalars in device memory. Every kernel returns at once when
+// the run is done, so the host reads the status once per chunk of iterations.
 #include <algorithm>
 #include <cmath>
-#include <climits>
 #include <cstring>
 #include <tuple>
-#include <type_traits>
 #include <utility>
-#include <vector>
 
+#include "krylov.cuh"
 #include "ops.cuh"
 #include "scan.cuh"
-#include "solver.cuh"
+#include "sell.cuh"
 
 namespace lsmps_gpu {
 
@@ -46,8 +42,9 @@ struct Partials {
 
 // Block sum of two doubles into partials[blockIdx]; returns true in the last block to
 // arrive, after which the caller may read all partials (fixed-order final sum).
+template <int NT = RB>
 __device__ __forceinline__ bool block_partials(double va, double vb, Partials P, unsigned int* counter) {
-    __shared__ double sa[RB / 32], sb[RB / 32];
+    __shared__ double sa[NT / 32], sb[NT / 32];
     __shared__ bool last;
     va = warp_sum(va);
     vb = warp_sum(vb);
@@ -56,7 +53,7 @@ __device__ __forceinline__ bool block_partials(double va, double vb, Partials P,
     __syncthreads();
     if (threadIdx.x == 0) {
         double ta = 0, tb = 0;
-        for (int k = 0; k < RB / 32; ++k) { ta += sa[k]; tb += sb[k]; }
+        for (int k = 0; k < NT / 32; ++k) { ta += sa[k]; tb += sb[k]; }
         P.a[blockIdx.x] = ta;
         P.b[blockIdx.x] = tb;
         __threadfence();
@@ -67,12 +64,13 @@ __device__ __forceinline__ bool block_partials(double va, double vb, Partials P,
     return last;
 }
 
-// In the last block: fixed-order sum of the partials (thread t sums entries t, t+RB, ...
+// In the last block: fixed-order sum of the partials (thread t sums entries t, t+NT, ...
 // then a fixed tree), result in *ra / *rb for thread 0.
+template <int NT = RB>
 __device__ __forceinline__ void final_sum(Partials P, double* ra, double* rb) {
-    __shared__ double sa[RB / 32], sb[RB / 32];
+    __shared__ double sa[NT / 32], sb[NT / 32];
     double va = 0, vb = 0;
-    for (int k = threadIdx.x; k < (int)gridDim.x; k += RB) {
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += NT) {
         va += __ldcg(P.a + k);
         vb += __ldcg(P.b + k);
     }
@@ -82,217 +80,20 @@ __device__ __forceinline__ void final_sum(Partials P, double* ra, double* rb) {
     __syncthreads();
     if (threadIdx.x == 0) {
         double ta = 0, tb = 0;
-        for (int k = 0; k < RB / 32; ++k) { ta += sa[k]; tb += sb[k]; }
+        for (int k = 0; k < NT / 32; ++k) { ta += sa[k]; tb += sb[k]; }
         *ra = ta;
         *rb = tb;
     }
 }
 
-// Row i of a SELL-32x4 matrix: slice s = i / 32 stores its 32 rows in chunks of four
-// consecutive entries per row (entries 4c..4c+3 of lane l at sptr[s] + 128 c + 4 l), zero-
-// padded to the slice's longest row rounded up to a multiple of four. One thread per row,
-// one warp per slice: each thread reads its next four values and four columns with two
-// 16-byte loads (a warp covers 512 contiguous bytes per load), and two chunks are issued
-// before their eight x gathers, so each thread keeps 64-96 bytes of matrix loads and eight
-// gathers in flight. Matrix loads stream past L1/L2 (__ldcs) so the vectors, re-read every
-// iteration, stay in the 126 MB L2.
-__device__ __forceinline__ void ld4(const float* p, float v[4]) {
-    float4 q = __ldcs(reinterpret_cast<const float4*>(p));
-    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-}
-__device__ __forceinline__ void ld4(const double* p, double v[4]) {
-    double2 a = __ldcs(reinterpret_cast<const double2*>(p));
-    double2 b = __ldcs(reinterpret_cast<const double2*>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-__device__ __forceinline__ void ld4(const int* p, int v[4]) {
-    int4 q = __ldcs(reinterpret_cast<const int4*>(p));
-    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-}
-// four 16-bit column steps (8 bytes) -> four columns continuing from c
-__device__ __forceinline__ void ld4_steps(const unsigned short* p, int& c, int out[4]) {
-    uint2 q = __ldcs(reinterpret_cast<const uint2*>(p));
-    c += (int)(q.x & 0xffffu);
-    out[0] = c;
-    c += (int)(q.x >> 16);
-    out[1] = c;
-    c += (int)(q.y & 0xffffu);
-    out[2] = c;
-    c += (int)(q.y >> 16);
-    out[3] = c;
-}
-
-// The row product with 16-bit column steps (2 bytes per entry instead of 4).
-template <class TM, class T>
-__device__ __forceinline__ double sell_row16(const Sell<TM>& A, long long s, int lane, const T* __restrict__ x) {
-    const long long base = (long long)A.sptr[s] + 4 * lane;
-    const TM* __restrict__ val = A.val + base;
-    const unsigned short* __restrict__ dc = A.dcol + base;
-    int cur = A.rbase[(s << 5) + lane];
-    const int chunks = A.slen[s] >> 2;
-    double a0 = 0, a1 = 0;
-    int c = 0;
-    for (; c + 2 <= chunks; c += 2) {
-        TM v0[4], v1[4];
-        int c0[4], c1[4];
-        ld4(val + 128 * c, v0);
-        ld4(val + 128 * (c + 1), v1);
-        ld4_steps(dc + 128 * c, cur, c0);
-        ld4_steps(dc + 128 * (c + 1), cur, c1);
-        T x0[4], x1[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            x0[j] = x[c0[j]];
-            x1[j] = x[c1[j]];
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            a0 += (double)v0[j] * (double)x0[j];
-            a1 += (double)v1[j] * (double)x1[j];
-        }
-    }
-    if (c < chunks) {
-        TM v0[4];
-        int c0[4];
-        ld4(val + 128 * c, v0);
-        ld4_steps(dc + 128 * c, cur, c0);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) a0 += (double)v0[j] * (double)x[c0[j]];
-    }
-    return a0 + a1;
-}
-
-// The same row product, software-pipelined: the next pair of chunks' values and column steps
-// are loaded while the current pair's gathers are in flight, so a pair of chunks waits for one
-// round trip instead of two. The sums are added in the same order as sell_row16 (same bits);
-// it needs ~64 registers, so its kernels run 4 blocks of RB threads per SM instead of 6.
-__device__ __forceinline__ void steps_to_cols(uint2 q, int& c, int out[4]) {
-    c += (int)(q.x & 0xffffu);
-    out[0] = c;
-    c += (int)(q.x >> 16);
-    out[1] = c;
-    c += (int)(q.y & 0xffffu);
-    out[2] = c;
-    c += (int)(q.y >> 16);
-    out[3] = c;
-}
-template <class TM, class T>
-__device__ __forceinline__ double sell_row16_pipe(const Sell<TM>& A, long long s, int lane,
-                                                  const T* __restrict__ x) {
-    const long long base = (long long)A.sptr[s] + 4 * lane;
-    const TM* __restrict__ val = A.val + base;
-    const unsigned short* __restrict__ dc = A.dcol + base;
-    int cur = A.rbase[(s << 5) + lane];
-    const int chunks = A.slen[s] >> 2;
-    double a0 = 0, a1 = 0;
-    int c = 0;
-    TM v0[4], v1[4];
-    uint2 s0 = make_uint2(0, 0), s1 = make_uint2(0, 0);
-    if (chunks >= 2) {
-        ld4(val, v0);
-        ld4(val + 128, v1);
-        s0 = __ldcs(reinterpret_cast<const uint2*>(dc));
-        s1 = __ldcs(reinterpret_cast<const uint2*>(dc + 128));
-    }
-    for (; c + 2 <= chunks; c += 2) {
-        int c0[4], c1[4];
-        steps_to_cols(s0, cur, c0);
-        steps_to_cols(s1, cur, c1);
-        T x0[4], x1[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            x0[j] = x[c0[j]];
-            x1[j] = x[c1[j]];
-        }
-        if (c + 4 <= chunks) {  // the next pair, in flight with the gathers above
-            TM w0[4], w1[4];
-            ld4(val + 128 * (c + 2), w0);
-            ld4(val + 128 * (c + 3), w1);
-            const uint2 t0 = __ldcs(reinterpret_cast<const uint2*>(dc + 128 * (c + 2)));
-            const uint2 t1 = __ldcs(reinterpret_cast<const uint2*>(dc + 128 * (c + 3)));
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                a0 += (double)v0[j] * (double)x0[j];
-                a1 += (double)v1[j] * (double)x1[j];
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                v0[j] = w0[j];
-                v1[j] = w1[j];
-            }
-            s0 = t0;
-            s1 = t1;
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                a0 += (double)v0[j] * (double)x0[j];
-                a1 += (double)v1[j] * (double)x1[j];
-            }
-        }
-    }
-    if (c < chunks) {
-        TM u0[4];
-        int c0[4];
-        ld4(val + 128 * c, u0);
-        ld4_steps(dc + 128 * c, cur, c0);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) a0 += (double)u0[j] * (double)x[c0[j]];
-    }
-    return a0 + a1;
-}
-
-// The solver SpMVs with FP32 values and 16-bit steps use the pipelined product.
-template <class TM, bool C16>
-constexpr bool sell_pipe() {
-    return C16 && sizeof(TM) == 4;
-}
+// grid of the row-product kernels: the pipelined products take 64 registers
 template <class TM, bool C16>
 constexpr int spmv_blocks_per_sm() {
-    return sell_pipe<TM, C16>() ? 4 : 6;
+    return C16 && sizeof(TM) == 4 ? 4 : 6;
 }
 template <class TM, bool C16>
 constexpr unsigned spmv_grid() {
     return 148u * spmv_blocks_per_sm<TM, C16>();
-}
-
-// C16: the view's columns are 16-bit steps (a compile-time choice: one code path per kernel)
-template <bool C16, class TM, class T>
-__device__ __forceinline__ double sell_row(const Sell<TM>& A, long long s, int lane, const T* __restrict__ x) {
-    if constexpr (C16) return sell_row16(A, s, lane, x);
-    const long long base = (long long)A.sptr[s] + 4 * lane;
-    const TM* __restrict__ val = A.val + base;
-    const int* __restrict__ col = A.col + base;
-    const int chunks = A.slen[s] >> 2;
-    double a0 = 0, a1 = 0;
-    int c = 0;
-    for (; c + 2 <= chunks; c += 2) {
-        TM v0[4], v1[4];
-        int c0[4], c1[4];
-        ld4(val + 128 * c, v0);
-        ld4(col + 128 * c, c0);
-        ld4(val + 128 * (c + 1), v1);
-        ld4(col + 128 * (c + 1), c1);
-        T x0[4], x1[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            x0[j] = x[c0[j]];
-            x1[j] = x[c1[j]];
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            a0 += (double)v0[j] * (double)x0[j];
-            a1 += (double)v1[j] * (double)x1[j];
-        }
-    }
-    if (c < chunks) {
-        TM v0[4];
-        int c0[4];
-        ld4(val + 128 * c, v0);
-        ld4(col + 128 * c, c0);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) a0 += (double)v0[j] * (double)x[c0[j]];
-    }
-    return a0 + a1;
 }
 
 #define SELL_LOOP(A)                                                              \
@@ -355,7 +156,7 @@ __global__ void __launch_bounds__(RB, spmv_blocks_per_sm<TM, C16>()) k_bcg_v(Sel
     if (S->done) return;
     double acc = 0;
     SELL_LOOP(A) {
-        double y = sell_pipe<TM, C16>() ? sell_row16_pipe(A, s, lane, p) : sell_row<C16>(A, s, lane, p);
+        double y = sell_product<C16>(A, s, lane, p);
         long long i = (s << 5) + lane;
         if (i < A.n) {
             T yi = (T)y;
@@ -510,27 +311,89 @@ __global__ void __launch_bounds__(RB) k_bcg_s_agg(MgFine G, const double* __rest
     }
 }
 
-// t = A sv; omega = (t, s) / (t, t), with sv = s, or the preconditioned M s when a
-// preconditioner is applied (s then only enters the dot)
+// t = A s; omega = (t, s) / (t, t)
 template <class T, class TM = T, bool C16 = false>
 __global__ void __launch_bounds__(RB, spmv_blocks_per_sm<TM, C16>()) k_bcg_t(Sell<TM> A, const T* __restrict__ sv, T* __restrict__ t,
-                                              BcgScalars* S, Partials P, const T* __restrict__ sd) {
+                                              BcgScalars* S, Partials P) {
     pdl_begin();
     if (S->done || S->s_conv) return;
     double ats = 0, att = 0;
     SELL_LOOP(A) {
-        double y = sell_pipe<TM, C16>() ? sell_row16_pipe(A, s, lane, sv) : sell_row<C16>(A, s, lane, sv);
+        double y = sell_product<C16>(A, s, lane, sv);
         long long i = (s << 5) + lane;
         if (i < A.n) {
             T ti = (T)y;
             t[i] = ti;
-            ats += (double)ti * (double)sd[i];
+            ats += (double)ti * (double)sv[i];
             att += (double)ti * (double)ti;
         }
     }
     if (block_partials(ats, att, P, &S->counter[2])) {
         double ts, tt;
         final_sum(P, &ts, &tt);
+        if (threadIdx.x == 0) {
+            S->counter[2] = 0;
+            S->tt = tt;
+            if (!isfinite(tt) || !isfinite(ts)) { S->nonfinite = 1; S->done = 2; }
+            else if (tt < 1e-30) S->done = 2;
+            else S->omega = ts / tt;
+        }
+    }
+}
+
+// The row products of the multigrid's iteration: one block of 1,024 threads per SM over a
+// contiguous run of slices (cut[b] .. cut[b + 1], about the same stored entries each), so that an
+// SM's gathers share lines in its L1. sd: t = A sv with the preconditioned sv = M s, whose dot takes s itself.
+constexpr int MGT = 1024;
+template <bool C16>
+__global__ void __launch_bounds__(MGT, 1) k_mg_v(Sell<float> A, const int* __restrict__ cut, const double* __restrict__ p,
+                                                 double* __restrict__ v, const double* __restrict__ r0, BcgScalars* S,
+                                                 Partials P) {
+    const int lane = threadIdx.x & 31, s1 = cut[blockIdx.x + 1];
+    int s = cut[blockIdx.x] + (threadIdx.x >> 5);  // (written before the solve)
+    pdl_begin();
+    if (S->done) return;
+    double acc = 0;
+    for (; s < s1; s += MGT / 32) {
+        const double y = sell_product<C16>(A, s, lane, p);
+        const long long i = ((long long)s << 5) + lane;
+        if (i < A.n) {
+            v[i] = y;
+            acc += r0[i] * y;
+        }
+    }
+    if (block_partials<MGT>(acc, 0.0, P, &S->counter[0])) {
+        double den, unused;
+        final_sum<MGT>(P, &den, &unused);
+        if (threadIdx.x == 0) {
+            S->counter[0] = 0;
+            if (!isfinite(den)) { S->nonfinite = 1; S->done = 2; }
+            else if (fabs(den) < 1e-30) S->done = 2;
+            else S->alpha = S->rho / den;
+        }
+    }
+}
+template <bool C16>
+__global__ void __launch_bounds__(MGT, 1) k_mg_t(Sell<float> A, const int* __restrict__ cut, const double* __restrict__ sv,
+                                                 double* __restrict__ t, const double* __restrict__ sd, BcgScalars* S,
+                                                 Partials P) {
+    const int lane = threadIdx.x & 31, s1 = cut[blockIdx.x + 1];
+    int s = cut[blockIdx.x] + (threadIdx.x >> 5);
+    pdl_begin();
+    if (S->done || S->s_conv) return;
+    double ats = 0, att = 0;
+    for (; s < s1; s += MGT / 32) {
+        const double y = sell_product<C16>(A, s, lane, sv);
+        const long long i = ((long long)s << 5) + lane;
+        if (i < A.n) {
+            t[i] = y;
+            ats += y * sd[i];
+            att += y * y;
+        }
+    }
+    if (block_partials<MGT>(ats, att, P, &S->counter[2])) {
+        double ts, tt;
+        final_sum<MGT>(P, &ts, &tt);
         if (threadIdx.x == 0) {
             S->counter[2] = 0;
             S->tt = tt;
@@ -618,9 +481,7 @@ template <class T, class TM = T, bool C16 = false>
 __global__ void __launch_bounds__(RB, 6) k_bcg_init(Sell<TM> A, const T* __restrict__ b, const T* __restrict__ x,
                                                  int use_x, T* __restrict__ r, T* __restrict__ r0,
                                                  T* __restrict__ p, T* __restrict__ v, BcgScalars* S,
-                                                 Partials P, double tol, double bnorm_override,
-                                                 const int* gate = nullptr, int want = 0) {
-    if (gate && *gate != want) return;  // device-driven loop: runs only when the control chose it
+                                                 Partials P, double tol, double bnorm_override) {
     double abb = 0, arr = 0;
     SELL_LOOP(A) {
         double ax = use_x ? sell_row<C16>(A, s, lane, x) : 0.0;
@@ -801,6 +662,14 @@ __global__ void __launch_bounds__(128) k_sell_build(long long n, long long nslic
 
 
 
+// cut[b]: the first slice of block b of SELL_CUTS, so that the blocks hold about the same number
+// of stored entries
+template <class T>
+__global__ void k_sell_cuts(Sell<T> A, int* __restrict__ cut) {
+    const int b = threadIdx.x;
+    if (b <= SELL_CUTS) cut[b] = (int)sell_cut(A, b, SELL_CUTS);
+}
+
 // ---------------------------------------------------------------------------------------
 // Mixed-precision helpers
 // ---------------------------------------------------------------------------------------
@@ -905,8 +774,7 @@ template <bool C16 = false>
 __global__ void __launch_bounds__(RB, 6) k_replace_residual(Sell<double> A, const double* __restrict__ b,
                                                             const double* __restrict__ y, double* __restrict__ r,
                                                             const double* __restrict__ r0, BcgScalars* S,
-                                                            Partials P, const int* gate = nullptr, int want = 0) {
-    if (gate && *gate != want) return;  // device-driven loop: runs only when the control chose it
+                                                            Partials P) {
     double arr = 0, ar0r = 0;
     SELL_LOOP(A) {
         double ay = sell_row<C16>(A, s, lane, y);
@@ -995,109 +863,6 @@ __global__ void k_solution_to_particles(long long U, const int* __restrict__ sor
 }
 
 // ---------------------------------------------------------------------------------------
-// device-driven solve loop: the host loop's decisions (residual replacement, restart, stop)
-// made by single-thread kernels between the iteration chunks of a conditional WHILE graph
-// node, so that a whole solve is one graph launch with no host round trip
-// ---------------------------------------------------------------------------------------
-struct LoopCtl {
-    double rn_upd;      // |r| at the last replacement or restart
-    double delta;       // replacement when |r| fell below delta rn_upd
-    int total;          // iterations so far (over restarts)
-    int base;           // S->iters at the last accounting
-    int replacements, restarts, fallback;
-    int act;            // 0 none, 1 replace, 2 restart: gates the replacement and init kernels
-    int final_replace;  // the pending replacement ends the solve (iteration cap)
-    int state;          // 0 running, 1 converged, 2 failed, 3 iteration cap, 4 multigrid gave up
-    int trips, max_trips, max_iter, use_nn;
-    int use_mg;         // the body applies the multigrid: a breakdown or stall ends it (state 4)
-    int stall;          // stall window of the restarted runs (multigrid only)
-};
-
-// as set_scalar_caps on the host: a fresh scalar block with the remaining iteration budget
-__device__ void restart_caps(BcgScalars* S, int max_iter, int stall) {
-    BcgScalars z{};
-    z.max_iter = max_iter;
-    z.stall_window = stall;
-    *S = z;
-}
-
-__global__ void k_mix_after_chunk(BcgScalars* S, LoopCtl* C) {
-    C->total += S->iters - C->base;
-    C->base = S->iters;
-    C->act = 0;
-    if (!S->done && S->rn > C->delta * C->rn_upd) return;  // keep iterating
-    const int why = S->done;
-    if (why == 3 || C->total >= C->max_iter) {
-        C->act = 1;
-        C->final_replace = 1;
-        return;
-    }
-    if (why == 0) {
-        C->act = 1;
-        C->final_replace = 0;
-        return;
-    }
-    if (C->use_mg && (why == 2 || why == 4)) {  // the multigrid broke down or stalled: host falls back
-        C->state = 4;
-        return;
-    }
-    if (why == 4 && C->use_nn) C->fallback = 1;
-    if (S->nonfinite) {
-        C->state = 2;
-        return;
-    }
-    restart_caps(S, C->max_iter - C->total, C->stall);
-    C->act = 2;
-}
-
-__global__ void k_mix_after_replace(BcgScalars* S, LoopCtl* C) {
-    if (C->act != 1) return;
-    C->act = 0;
-    if (C->final_replace) {
-        C->state = S->done == 1 ? 1 : 3;
-        return;
-    }
-    C->replacements += 1;
-    C->rn_upd = S->rn;
-    if (S->done == 1) {
-        C->state = 1;
-        return;
-    }
-    if (S->done == 0) return;
-    if (C->use_mg) {  // breakdown after the replacement with the multigrid: host falls back
-        C->state = 4;
-        return;
-    }
-    if (S->nonfinite) {  // breakdown after the replacement: restart, unless non-finite
-        C->state = 2;
-        return;
-    }
-    restart_caps(S, C->max_iter - C->total, C->stall);
-    C->act = 2;
-}
-
-__global__ void k_mix_after_restart(BcgScalars* S, LoopCtl* C) {
-    if (C->act != 2) return;
-    C->act = 0;
-    C->restarts += 1;
-    C->base = 0;
-    C->rn_upd = S->rn;
-    if (S->done == 1) C->state = 1;
-    else if (S->done) C->state = 2;
-}
-
-// plain loop (FP64 / Jacobi): stop when the iteration stopped
-__global__ void k_plain_after_chunk(const BcgScalars* S, LoopCtl* C) {
-    if (S->done) C->state = S->done == 1 ? 1 : 2;
-}
-
-// the WHILE condition; trips are bounded whatever the control state says
-__global__ void k_loop_continue(LoopCtl* C, cudaGraphConditionalHandle h) {
-    C->trips += 1;
-    cudaGraphSetConditional(h, (C->state == 0 && C->trips < C->max_trips) ? 1u : 0u);
-}
-
-// ---------------------------------------------------------------------------------------
 // host side of the engine
 // ---------------------------------------------------------------------------------------
 struct Engine {
@@ -1123,90 +888,37 @@ Engine make_engine(lsmps_ctx* ctx) {
 
 double* engine_scalars(lsmps_ctx* ctx) { return ctx->red.get<double>() + 2 * RGRID + 128; }
 
-LoopCtl* engine_loop_ctl(lsmps_ctx* ctx) {
-    return reinterpret_cast<LoopCtl*>(ctx->red.get<double>() + 2 * RGRID + 160);
-}
-static_assert(sizeof(BcgScalars) <= 128 * sizeof(double) && sizeof(LoopCtl) <= 96 * sizeof(double),
-              "engine scalar layout");
+static_assert(sizeof(BcgScalars) <= 128 * sizeof(double), "engine scalar layout");
 
-// A graph whose one node is a WHILE conditional: its body (captured from stream s by `body`,
-// then k_loop_continue) runs until the control clears the condition.
-template <class F>
-cudaGraphExec_t build_while_graph(cudaStream_t s, LoopCtl* C, F&& body) {
-    cudaGraph_t g = nullptr;
-    LSMPS_CUDA(cudaGraphCreate(&g, 0));
-    cudaGraphExec_t exec = nullptr;
-    try {
-        cudaGraphConditionalHandle h;
-        LSMPS_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
-        cudaGraphNodeParams np{};
-        np.type = cudaGraphNodeTypeConditional;
-        np.conditional.handle = h;
-        np.conditional.type = cudaGraphCondTypeWhile;
-        np.conditional.size = 1;
-        cudaGraphNode_t node;
-        LSMPS_CUDA(cudaGraphAddNode(&node, g, nullptr, 0, &np));
-        LSMPS_CUDA(cudaStreamBeginCaptureToGraph(s, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                                 cudaStreamCaptureModeThreadLocal));
-        body();
-        k_loop_continue<<<1, 1, 0, s>>>(C, h);
-        cudaGraph_t captured = nullptr;
-        LSMPS_CUDA(cudaStreamEndCapture(s, &captured));
-        LSMPS_CUDA(cudaGraphInstantiate(&exec, g, 0));
-    } catch (...) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
-            cudaGraph_t tmp = nullptr;
-            cudaStreamEndCapture(s, &tmp);
-            if (tmp) cudaGraphDestroy(tmp);
-        }
-        cudaGetLastError();
-        cudaGraphDestroy(g);
-        throw;
-    }
-    cudaGraphDestroy(g);
-    return exec;
-}
-
-// One BiCGStab iteration; with `mg` (FP64 vectors only) the multigrid V-cycle is the right
-// preconditioner: ph = D M p before v = A ph, sh = D M s before t = A sh.
-template <class T, class TM = T>
-void iteration(Engine& E, const Sell<TM>& A, const Vecs<T>& V, bool mg = false) {
+// One BiCGStab iteration (MIXED_F32)
+template <class T>
+void iteration(Engine& E, const Sell<T>& A, const Vecs<T>& V) {
     note_launches(5);
-    const T* pv = V.p;
-    const T* sv = V.s;
-    if constexpr (std::is_same<T, double>::value) {
-        if (mg) {  // p and its level-1 restriction in one pass, then the rest of the V-cycle
-            const MgFine G = mg_fine(E.ctx);
-            launch_pdl(k_bcg_p_agg, agg_blocks(G.n1), RB, 0, E.s, G, V.r, V.p, V.v, E.S);
-            mg_apply(E.ctx, V.p, V.ph, E.S, 0, true);
-            pv = V.ph;
-        }
-    }
-    if (!mg) launch_pdl(k_bcg_p<T>, RGRID, RB, 0, E.s, A.n, V.r, V.p, V.v, E.S);
-    if (A.dcol) launch_pdl(k_bcg_v<T, TM, true>, spmv_grid<TM, true>(), RB, 0, E.s, A, pv, V.v, V.r0, E.S, E.P);
-    else launch_pdl(k_bcg_v<T, TM, false>, RGRID, RB, 0, E.s, A, pv, V.v, V.r0, E.S, E.P);
-    if constexpr (std::is_same<T, double>::value) {
-        if (mg) {
-            const MgFine G = mg_fine(E.ctx);
-            launch_pdl(k_bcg_s_agg, std::min<unsigned>(RGRID, agg_blocks(G.n1)), RB, 0, E.s, G, V.r, V.v, V.s, E.S,
-                       E.P);
-            mg_apply(E.ctx, V.s, V.sh, E.S, 1, true);
-            sv = V.sh;
-        }
-    }
-    if (!mg) launch_pdl(k_bcg_s<T>, RGRID, RB, 0, E.s, A.n, V.r, V.v, V.s, E.S, E.P);
-    if (A.dcol) launch_pdl(k_bcg_t<T, TM, true>, spmv_grid<TM, true>(), RB, 0, E.s, A, sv, V.t, E.S, E.P, V.s);
-    else launch_pdl(k_bcg_t<T, TM, false>, RGRID, RB, 0, E.s, A, sv, V.t, E.S, E.P, V.s);
-    if (mg)
-        launch_pdl(k_bcg_x<T, true>, RGRID, RB, 0, E.s, A.n, V.x, V.r, V.p, V.s, V.t, V.r0, E.S, E.P, V.ph, V.sh);
-    else
-        launch_pdl(k_bcg_x<T, false>, RGRID, RB, 0, E.s, A.n, V.x, V.r, V.p, V.s, V.t, V.r0, E.S, E.P,
-                   (const T*)nullptr, (const T*)nullptr);
+    launch_pdl(k_bcg_p<T>, RGRID, RB, 0, E.s, A.n, V.r, V.p, V.v, E.S);
+    if (A.dcol) launch_pdl(k_bcg_v<T, T, true>, spmv_grid<T, true>(), RB, 0, E.s, A, V.p, V.v, V.r0, E.S, E.P);
+    else launch_pdl(k_bcg_v<T, T, false>, RGRID, RB, 0, E.s, A, V.p, V.v, V.r0, E.S, E.P);
+    launch_pdl(k_bcg_s<T>, RGRID, RB, 0, E.s, A.n, V.r, V.v, V.s, E.S, E.P);
+    if (A.dcol) launch_pdl(k_bcg_t<T, T, true>, spmv_grid<T, true>(), RB, 0, E.s, A, V.s, V.t, E.S, E.P);
+    else launch_pdl(k_bcg_t<T, T, false>, RGRID, RB, 0, E.s, A, V.s, V.t, E.S, E.P);
+    launch_pdl(k_bcg_x<T, false>, RGRID, RB, 0, E.s, A.n, V.x, V.r, V.p, V.s, V.t, V.r0, E.S, E.P, (const T*)nullptr,
+               (const T*)nullptr);
 }
 
-// kernel launches of one iteration
-int launches_per_iteration(lsmps_ctx* ctx, bool mg) { return 5 + (mg ? 2 * mg_launches_per_apply(ctx, true) : 0); }
+// One iteration with the multigrid V-cycle as the right preconditioner: p (and s) and its
+// level-1 restriction in one pass, the rest of the V-cycle, then the row product.
+void iteration_mg(Engine& E, const Sell<float>& A, const Vecs<double>& V, const int* cut) {
+    note_launches(5);
+    const MgFine G = mg_fine(E.ctx);
+    launch_pdl(k_bcg_p_agg, agg_blocks(G.n1), RB, 0, E.s, G, V.r, V.p, V.v, E.S);
+    mg_apply(E.ctx, V.p, V.ph, E.S, 0, true);
+    if (A.dcol) launch_pdl(k_mg_v<true>, SELL_CUTS, MGT, 0, E.s, A, cut, V.ph, V.v, V.r0, E.S, E.P);
+    else launch_pdl(k_mg_v<false>, SELL_CUTS, MGT, 0, E.s, A, cut, V.ph, V.v, V.r0, E.S, E.P);
+    launch_pdl(k_bcg_s_agg, std::min<unsigned>(RGRID, agg_blocks(G.n1)), RB, 0, E.s, G, V.r, V.v, V.s, E.S, E.P);
+    mg_apply(E.ctx, V.s, V.sh, E.S, 1, true);
+    if (A.dcol) launch_pdl(k_mg_t<true>, SELL_CUTS, MGT, 0, E.s, A, cut, V.sh, V.t, V.s, E.S, E.P);
+    else launch_pdl(k_mg_t<false>, SELL_CUTS, MGT, 0, E.s, A, cut, V.sh, V.t, V.s, E.S, E.P);
+    launch_pdl(k_bcg_x<double, true>, RGRID, RB, 0, E.s, A.n, V.x, V.r, V.p, V.s, V.t, V.r0, E.S, E.P, V.ph, V.sh);
+}
 
 template <class T, class TM = T>
 void init(Engine& E, const Sell<TM>& A, const T* b, const Vecs<T>& V, bool use_x, double tol, double bnorm_override) {
@@ -1219,75 +931,17 @@ void init(Engine& E, const Sell<TM>& A, const T* b, const Vecs<T>& V, bool use_x
     LSMPS_CHECK_LAUNCH();
 }
 
-// the mixed solver's FP64 residual replacement (gated by the device-driven loop's control)
-void launch_replace(cudaStream_t s, const Sell<double>& As, const double* b, const Vecs<double>& V, Engine& E,
-                    const int* gate, int want) {
-    if (As.dcol) k_replace_residual<true><<<RGRID, RB, 0, s>>>(As, b, V.x, V.r, V.r0, E.S, E.P, gate, want);
-    else k_replace_residual<false><<<RGRID, RB, 0, s>>>(As, b, V.x, V.r, V.r0, E.S, E.P, gate, want);
+// the mixed solver's FP64 residual replacement
+void launch_replace(cudaStream_t s, const Sell<double>& As, const double* b, const Vecs<double>& V, Engine& E) {
+    if (As.dcol) k_replace_residual<true><<<RGRID, RB, 0, s>>>(As, b, V.x, V.r, V.r0, E.S, E.P);
+    else k_replace_residual<false><<<RGRID, RB, 0, s>>>(As, b, V.x, V.r, V.r0, E.S, E.P);
+    LSMPS_CHECK_LAUNCH();
 }
 
 void residual64(Engine& E, const Sell<double>& A, const double* b, const double* x, double* r, double* out2) {
     if (A.dcol) k_residual64<true><<<RGRID, RB, 0, E.s>>>(A, b, x, r, out2, E.P, &E.S->counter[5]);
     else k_residual64<false><<<RGRID, RB, 0, E.s>>>(A, b, x, r, out2, E.P, &E.S->counter[5]);
     LSMPS_CHECK_LAUNCH();
-}
-
-// Runs the iteration until done. mode 1: one graph whose WHILE node repeats `chunk`
-// iterations until the scalars say done (no host round trip); mode 2: a graph of `chunk`
-// iterations launched from a host loop that reads the scalars after each; mode 0: eager
-// launches with the same host loop. Returns the final scalars.
-template <class T>
-BcgScalars run_loop(Engine& E, const Sell<T>& A, const Vecs<T>& V, int chunk, int mode) {
-    BcgScalars h{};
-    LSMPS_CUDA(cudaMemcpyAsync(&h, E.S, sizeof(h), cudaMemcpyDeviceToHost, E.s));
-    LSMPS_CUDA(cudaStreamSynchronize(E.s));
-    // the iteration cap bounds the loop; two extra chunks cover the final no-op kernels
-    const long long max_chunks = (h.max_iter + chunk - 1) / chunk + 2;
-    if (h.done) return h;
-    if (mode == 1) {
-        LoopCtl* C = engine_loop_ctl(E.ctx);
-        LoopCtl c0{};
-        c0.max_trips = (int)std::min<long long>(max_chunks, INT_MAX);
-        LSMPS_CUDA(cudaMemcpyAsync(C, &c0, sizeof(c0), cudaMemcpyHostToDevice, E.s));
-        cudaGraphExec_t exec = build_while_graph(E.s, C, [&] {
-            for (int c = 0; c < chunk; ++c) iteration<T>(E, A, V);
-            k_plain_after_chunk<<<1, 1, 0, E.s>>>(E.S, C);
-        });
-        note_launches(0 - (uint64_t)(5 * chunk));  // captured, not launched
-        cudaError_t e = cudaGraphLaunch(exec, E.s);
-        LoopCtl hc{};
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&hc, C, sizeof(hc), cudaMemcpyDeviceToHost, E.s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&h, E.S, sizeof(h), cudaMemcpyDeviceToHost, E.s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(E.s);
-        cudaGraphExecDestroy(exec);
-        LSMPS_CUDA(e);
-        note_launches((uint64_t)hc.trips * (5 * (uint64_t)chunk + 2));
-        return h;
-    }
-    cudaGraphExec_t exec = nullptr;
-    if (mode == 2) {
-        cudaGraph_t graph;
-        LSMPS_CUDA(cudaStreamBeginCapture(E.s, cudaStreamCaptureModeThreadLocal));
-        for (int c = 0; c < chunk; ++c) iteration<T>(E, A, V);
-        note_launches(0 - (uint64_t)(5 * chunk));  // captured, not launched
-        cudaError_t e = cudaStreamEndCapture(E.s, &graph);
-        LSMPS_CUDA(e);
-        LSMPS_CUDA(cudaGraphInstantiate(&exec, graph, 0));
-        cudaGraphDestroy(graph);
-    }
-    for (long long c = 0; c < max_chunks && !h.done; ++c) {
-        if (exec) {
-            LSMPS_CUDA(cudaGraphLaunch(exec, E.s));
-            note_launches(5 * (uint64_t)chunk);
-        } else {
-            for (int k = 0; k < chunk; ++k) iteration<T>(E, A, V);
-            LSMPS_CHECK_LAUNCH();
-        }
-        LSMPS_CUDA(cudaMemcpyAsync(&h, E.S, sizeof(h), cudaMemcpyDeviceToHost, E.s));
-        LSMPS_CUDA(cudaStreamSynchronize(E.s));
-    }
-    if (exec) cudaGraphExecDestroy(exec);
-    return h;
 }
 
 void set_scalar_caps(Engine& E, int max_iter, int stall_window) {
@@ -1362,6 +1016,14 @@ static void sell_raw(lsmps_ctx* ctx) {
 }
 
 template <class T>
+static const int* sell_cuts(lsmps_ctx* ctx, const Sell<T>& A) {
+    int* cut = ctx->S_cut.ensure<int>(SELL_CUTS + 1);
+    k_sell_cuts<<<1, 256, 0, ctx->stream>>>(A, cut);
+    LSMPS_CHECK_LAUNCH();
+    return cut;
+}
+
+template <class T>
 static Sell<T> sell_view(lsmps_ctx* ctx, const T* val) {
     Sell<T> A{ctx->U, ctx->sell_nslices, ctx->S_ptr.get<int>(), ctx->S_len.get<int>(), ctx->S_col.get<int>(), val};
     if (ctx->have_steps) {
@@ -1391,38 +1053,47 @@ static Sell<float> sell_scaled32(lsmps_ctx* ctx) {  // A D^-1 in FP32 (built wit
 
 Sell<float> sell_scaled32_view(lsmps_ctx* ctx) { return sell_scaled32(ctx); }
 
+static KrylovVecs krylov_vecs(lsmps_ctx* ctx) {
+    const long long U = ctx->U;
+    KrylovVecs V{ctx->vx.ensure<double>(U + 2), ctx->vr.ensure<double>(U + 2), ctx->vr0.ensure<double>(U + 2),
+                 ctx->vp.ensure<double>(U + 2), ctx->vv.ensure<double>(U + 2), ctx->vs.ensure<double>(U + 2),
+                 ctx->vt.ensure<double>(U + 2)};
+    V.b = ctx->A_b.get<double>();
+    return V;
+}
+
+static void krylov_stats(lsmps_ctx* ctx, const KrylovResult& h, lsmps_ppe_stats* ps) {
+    double mx;
+    std::memcpy(&mx, &h.maxbits, sizeof(mx));
+    ps->iterations = h.iterations;
+    ps->outer_iterations = h.outer;
+    ps->converged = h.converged && !h.nonfinite;
+    ps->fallback = h.fallback;
+    ps->max_error = mx;
+    ps->relative_l2_error = std::sqrt(h.err2 / std::max(h.ref2, 1e-30));
+    ps->solve_ms = ev_elapsed(ctx, 10, 11);
+}
+
 // Fast FP64 / Jacobi: BiCGStab on A (or A D^-1) in FP64.
 static void solve_fast64(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_stats* ps, bool jacobi) {
-    cudaStream_t s = ctx->stream;
-    long long U = ctx->U;
-    Engine E = make_engine(ctx);
-    Vecs<double> V{ctx->vx.ensure<double>(U + 1), ctx->vr.ensure<double>(U + 1), ctx->vr0.ensure<double>(U + 1),
-                   ctx->vp.ensure<double>(U + 1), ctx->vv.ensure<double>(U + 1), ctx->vs.ensure<double>(U + 1),
-                   ctx->vt.ensure<double>(U + 1)};
-    const double* dinv = ctx->A_dinv.get<double>();
-    bool warm = o->warm_start && ctx->have_solution;
+    const long long U = ctx->U;
+    const bool warm = o->warm_start && ctx->have_solution;
     ev_record(ctx, 10);
-    Sell<double> Aop = jacobi ? sell_scaled64(ctx) : sell_a64(ctx);
-    set_scalar_caps(E, o->max_iter, 0);
+    const KrylovVecs V = krylov_vecs(ctx);
+    const Sell<double> A = jacobi ? sell_scaled64(ctx) : sell_a64(ctx);
+    const double* dinv = ctx->A_dinv.get<double>();
     if (warm && jacobi) {  // the iteration works on y = D x
-        k_scale_by_diag<<<1184, 256, 0, s>>>(U, V.x, dinv);
-        LSMPS_CHECK_LAUNCH();
-    } else if (!warm) {
-        LSMPS_CUDA(cudaMemsetAsync(V.x, 0, U * sizeof(double), s));
-    }
-    init<double>(E, Aop, ctx->A_b.get<double>(), V, warm, o->tol, -1.0);
-    int chunk = std::max(1, o->check_every > 0 ? o->check_every : 8);
-    BcgScalars h = run_loop<double>(E, Aop, V, chunk, o->use_graph);
-    if (jacobi) {
-        k_unscale<<<1184, 256, 0, s>>>(U, V.x, dinv);
+        k_scale_by_diag<<<1184, 256, 0, ctx->stream>>>(U, V.x, dinv);
         LSMPS_CHECK_LAUNCH();
     }
-    ev_record(ctx, 11);
-    LSMPS_CUDA(cudaStreamSynchronize(s));
-    ps->iterations = h.iters;
-    ps->converged = h.done == 1;
-    ps->solve_ms = ev_elapsed(ctx, 10, 11);
-    if (h.nonfinite) ps->converged = 0;
+    KrylovOpts k;
+    k.tol = o->tol;
+    k.chunk = std::max(1, o->check_every > 0 ? o->check_every : 8);
+    k.max_iter = o->max_iter;
+    k.use_x = warm;
+    k.dinv = jacobi ? dinv : nullptr;
+    k.xe = ctx->A_xexact.get<double>();
+    krylov_stats(ctx, krylov_solve(ctx, nullptr, A, V, k), ps);
 }
 
 // Mixed precision with FP32 vectors (MIXED_F32). One FP32 Jacobi-BiCGStab on A D^-1 y = r0 / sigma (sigma =
@@ -1442,7 +1113,7 @@ static void solve_mixed_f32(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_pp
     double* scal = engine_scalars(ctx);  // [0] |r|^2, [1] |b|^2, [6] sigma
     double* sigma = scal + 6;
     const double* dinv = ctx->A_dinv.get<double>();
-    double* x = ctx->vx.ensure<double>(U + 1);
+    double* x = ctx->vx.ensure<double>(U + 2);
     double* r64 = ctx->vr.ensure<double>(U + 1);
     float* rhs = ctx->fph.ensure<float>(U + 1);
     Vecs<float> V{ctx->fx.ensure<float>(U + 1), ctx->fr.ensure<float>(U + 1), ctx->fr0.ensure<float>(U + 1),
@@ -1588,30 +1259,33 @@ static void side_stream_fork(lsmps_ctx* ctx) {
 // Jacobi-BiCGStab (fallback). With the multigrid preconditioner a stall (no 1 % progress in
 // `stall_window` iterations) or a breakdown ends the multigrid phase, and the solve continues
 // as Jacobi MIXED from the current iterate (from zero when it is no longer finite; fallback).
-// exit_res (optional): {|b - A D^-1 y|, |b|} of the returned iterate when the solve converged
-// (the convergence test's own FP64 residual), else {-1, -1}.
-static void solve_mixed(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_stats* ps, bool learned,
-                        double* exit_res = nullptr) {
+// exit_res: {|b - A D^-1 y|, |b|} of the returned iterate when the solve converged (the
+// convergence test's own FP64 residual), else {-1, -1}. Returns whether ps holds the error
+// against p*. The Jacobi solves run in krylov.cu's one launch; the multigrid's launch the
+// iteration's kernels from the host, 2 x 11 + 5 of them, each under programmatic dependent launch
+// (the same steps between the grid barriers of one launch measured 370-400 against 290 us per
+// iteration at 1M: one block of 1,024 threads per SM hides less of the V-cycle's dependent
+// loads than the kernels' 2,048 threads, and its shared memory takes the L1 from the row products).
+static bool solve_mixed(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_stats* ps, bool learned,
+                        double* exit_res) {
     cudaStream_t s = ctx->stream;
     const long long U = ctx->U;
-    Engine E = make_engine(ctx);
     const double* dinv = ctx->A_dinv.get<double>();
     const double* b = ctx->A_b.get<double>();
-    Vecs<double> V{ctx->vx.ensure<double>(U + 1), ctx->vr.ensure<double>(U + 1), ctx->vr0.ensure<double>(U + 1),
-                   ctx->vp.ensure<double>(U + 1), ctx->vv.ensure<double>(U + 1), ctx->vs.ensure<double>(U + 1),
-                   ctx->vt.ensure<double>(U + 1)};
     const bool use_nn = learned && mpnn_ready(ctx);
     const bool warm = o->warm_start && ctx->have_solution;
-    const double delta = o->inner_tol > 0 ? o->inner_tol : 0.01;
-    const int chunk = std::max(1, o->check_every > 0 ? o->check_every : 8);
+    const bool mg = o->precond == LSMPS_PRECOND_MULTIGRID;
     const int stall = o->stall_window > 0 ? o->stall_window : 20;
     ev_record(ctx, 10);
-    const bool mg = o->precond == LSMPS_PRECOND_MULTIGRID;
+    const KrylovVecs K = krylov_vecs(ctx);
+    Vecs<double> V{K.x, K.r, K.r0, K.p, K.v, K.s, K.t};
+    Engine E = make_engine(ctx);
+    double* scal = engine_scalars(ctx);
+    if (use_nn) set_scalar_caps(E, 0, 0);  // zeroes the reduction tickets of the kernels below
     // y0 = |b| net(b / |b|): launches only (no host round trip)
     auto net_guess = [&] {
         float* rhs = ctx->fph.ensure<float>(U + 1);
         float* yf = ctx->fx.ensure<float>(U + 1);
-        double* scal = engine_scalars(ctx);
         k_norm2<<<RGRID, RB, 0, s>>>(U, b, scal, E.P, &E.S->counter[5]);
         k_rhs_unit<<<1184, 256, 0, s>>>(U, b, rhs, scal);  // network input: b / |b| in FP32
         LSMPS_CHECK_LAUNCH();
@@ -1634,205 +1308,139 @@ static void solve_mixed(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_st
         V.ph = ctx->vph.ensure<double>(U + 1);
         V.sh = ctx->vsh.ensure<double>(U + 1);
     }
-    Sell<double> As = sell_scaled64(ctx);
-    Sell<float> Af = sell_scaled32(ctx);
-    set_scalar_caps(E, o->max_iter, (use_nn || mg) ? stall : 0);
-    bool have_start = warm;
-    double warm_rn = 0;  // |b - A x0| of a warm start the network corrected
+    const Sell<double> As = sell_scaled64(ctx);
+    const Sell<float> Af = sell_scaled32(ctx);
+    KrylovOpts ko;
+    ko.tol = o->tol;
+    ko.delta = o->inner_tol > 0 ? o->inner_tol : 0.01;
+    ko.chunk = std::max(1, o->check_every > 0 ? o->check_every : 8);
+    ko.max_iter = o->max_iter;
+    ko.max_chunks = (long long)o->max_iter / ko.chunk + 4 + o->max_iter;
+    ko.stall = stall;
+    ko.use_x = warm || use_nn;
+    ko.use_nn = use_nn;
+    ko.dinv = dinv;
+    ko.xe = ctx->A_xexact.get<double>();
     if (warm) {  // the iteration works on y = D x
         k_scale_by_diag<<<1184, 256, 0, s>>>(U, V.x, dinv);
         LSMPS_CHECK_LAUNCH();
         if (use_nn) {  // the network corrects the warm start: y += |r0| net(r0 / |r0|), r0 = b - A D^-1 y
             float* rhs = ctx->fph.ensure<float>(U + 1);
             float* yf = ctx->fx.ensure<float>(U + 1);
-            double* scal = engine_scalars(ctx);
             residual64(E, As, b, V.x, V.r, scal);
             k_rhs_unit<<<1184, 256, 0, s>>>(U, V.r, rhs, scal);
             LSMPS_CHECK_LAUNCH();
             mpnn_warm_start(ctx, rhs, yf);
-            k_y_add_net<<<1184, 256, 0, s>>>(U, yf, scal, V.x, V.p);  // the warm start kept in p
+            k_y_add_net<<<1184, 256, 0, s>>>(U, yf, scal, V.x, V.s);  // the warm start kept in s
             LSMPS_CHECK_LAUNCH();
-            double r2 = 0;
-            LSMPS_CUDA(cudaMemcpyAsync(&r2, scal, sizeof(double), cudaMemcpyDeviceToHost, s));
-            LSMPS_CUDA(cudaStreamSynchronize(s));
-            warm_rn = std::sqrt(r2);
+            ko.warm_rn2 = scal;
         }
-    } else if (use_nn) {
-        if (!overlap) net_guess();
-        have_start = true;
-    } else {
-        LSMPS_CUDA(cudaMemsetAsync(V.x, 0, U * sizeof(double), s));
+    } else if (use_nn && !overlap) {
+        net_guess();
     }
-    init<double, double>(E, As, b, V, have_start, o->tol, -1.0);
-    auto read = [&](BcgScalars& h) {
-        LSMPS_CUDA(cudaMemcpyAsync(&h, E.S, sizeof(h), cudaMemcpyDeviceToHost, s));
-        LSMPS_CUDA(cudaStreamSynchronize(s));
+    exit_res[0] = exit_res[1] = -1.0;
+    auto finish = [&](const KrylovResult& h) {
+        krylov_stats(ctx, h, ps);
+        // convergence is only declared right after a residual replacement or a (re)start, whose
+        // FP64 residual b - A D^-1 y of the final iterate h holds
+        if (h.converged && std::isfinite(h.rn)) {
+            exit_res[0] = h.rn;
+            exit_res[1] = h.bnorm;
+        }
+        return true;
     };
-    BcgScalars h{};
-    read(h);
-    int total = 0, replacements = 0, restarts = 0, fallback = 0;
-    if (use_nn && !warm && (!std::isfinite(h.rn) || h.rn >= h.bnorm)) {
-        // the network's guess is worse than zero: discard it and run plain Jacobi-BiCGStab
-        fallback = 1;
-        LSMPS_CUDA(cudaMemsetAsync(V.x, 0, U * sizeof(double), s));
-        set_scalar_caps(E, o->max_iter, mg ? stall : 0);
-        init<double, double>(E, As, b, V, false, o->tol, -1.0);
-        read(h);
-    } else if (use_nn && warm && (!std::isfinite(h.rn) || h.rn >= warm_rn)) {
-        // the correction made the warm start worse: go back to it
-        fallback = 1;
-        LSMPS_CUDA(cudaMemcpyAsync(V.x, V.p, U * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        set_scalar_caps(E, o->max_iter, mg ? stall : 0);
-        init<double, double>(E, As, b, V, true, o->tol, -1.0);
-        read(h);
+    if (!mg) {
+        KrylovVecs W = K;
+        W.keep = V.s;
+        return finish(krylov_solve(ctx, &Af, As, W, ko));
     }
-    bool converged = h.done == 1, failed = h.done == 2 && h.nonfinite;
-    const long long max_chunks = (long long)o->max_iter / chunk + 4 + o->max_iter;  // bounded loop
-    // Iterates from the scalars in h until converged, failed or the iteration cap; with the
-    // multigrid (mgp), a breakdown or a stall ends the phase early and returns true instead
-    // (the caller then continues without it).
-    auto phase = [&](bool mgp) -> bool {
-        const uint64_t kpi = (uint64_t)launches_per_iteration(ctx, mgp);
-        const int restart_stall = mgp ? stall : 0;
-        double rn_upd = h.rn;
-        if (o->use_graph == 1) {
-            if (converged || failed) return false;
-            // the loop below, decided on the device: one graph launch for the whole solve
-            LoopCtl* C = engine_loop_ctl(ctx);
-            LoopCtl c0{};
-            c0.rn_upd = rn_upd;
-            c0.delta = delta;
-            c0.fallback = fallback;
-            c0.max_trips = (int)std::min<long long>(max_chunks, INT_MAX);
-            c0.max_iter = o->max_iter;
-            c0.total = total;
-            c0.use_nn = use_nn ? 1 : 0;
-            c0.use_mg = mgp ? 1 : 0;
-            c0.stall = restart_stall;
-            LSMPS_CUDA(cudaMemcpyAsync(C, &c0, sizeof(c0), cudaMemcpyHostToDevice, s));
-            cudaGraphExec_t wexec = build_while_graph(s, C, [&] {
-                for (int c = 0; c < chunk; ++c) iteration<double, float>(E, Af, V, mgp);
-                k_mix_after_chunk<<<1, 1, 0, s>>>(E.S, C);
-                launch_replace(s, As, b, V, E, &C->act, 1);
-                k_mix_after_replace<<<1, 1, 0, s>>>(E.S, C);
-                if (As.dcol)
-                    k_bcg_init<double, double, true><<<RGRID, RB, 0, s>>>(As, b, V.x, 1, V.r, V.r0, V.p, V.v, E.S,
-                                                                          E.P, o->tol, -1.0, &C->act, 2);
-                else
-                    k_bcg_init<double, double, false><<<RGRID, RB, 0, s>>>(As, b, V.x, 1, V.r, V.r0, V.p, V.v, E.S,
-                                                                           E.P, o->tol, -1.0, &C->act, 2);
-                k_mix_after_restart<<<1, 1, 0, s>>>(E.S, C);
-            });
-            note_launches(0 - kpi * (uint64_t)chunk);  // captured, not launched
-            cudaError_t e = cudaGraphLaunch(wexec, s);
-            LoopCtl hc{};
-            if (e == cudaSuccess) e = cudaMemcpyAsync(&hc, C, sizeof(hc), cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(&h, E.S, sizeof(h), cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-            cudaGraphExecDestroy(wexec);
-            LSMPS_CUDA(e);
-            note_launches((uint64_t)hc.trips * (kpi * (uint64_t)chunk + 6));
-            total = hc.total;
-            replacements += hc.replacements;
-            restarts += hc.restarts;
-            fallback = hc.fallback;
-            converged = hc.state == 1;
-            failed = hc.state == 2;
-            return hc.state == 4;
+    const int* cut = sell_cuts(ctx, Af);
+    set_scalar_caps(E, o->max_iter, stall);
+    if (!ko.use_x) LSMPS_CUDA(cudaMemsetAsync(V.x, 0, U * sizeof(double), s));
+    init<double, double>(E, As, b, V, ko.use_x != 0, o->tol, -1.0);
+    BcgScalars h{};
+    double warm_rn2 = 0;  // |b - A x0|^2 of a warm start the network corrected
+    auto read = [&] { read_back(ctx, {{E.S, &h, sizeof(h)}}, nullptr); };
+    read_back(ctx, {{E.S, &h, sizeof(h)}, {scal, &warm_rn2, sizeof(warm_rn2)}}, nullptr);
+    int total = 0, replacements = 0, restarts = 0, fallback = 0;
+    if (use_nn && (!std::isfinite(h.rn) || h.rn >= (warm ? std::sqrt(warm_rn2) : h.bnorm))) {
+        // the network's guess is worse than zero (its correction than the warm start): discard it
+        fallback = 1;
+        if (warm) LSMPS_CUDA(cudaMemcpyAsync(V.x, V.s, U * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        else LSMPS_CUDA(cudaMemsetAsync(V.x, 0, U * sizeof(double), s));
+        set_scalar_caps(E, o->max_iter, stall);
+        init<double, double>(E, As, b, V, warm, o->tol, -1.0);
+        read();
+    }
+    // iterates until converged, failed or the iteration cap, or until the multigrid breaks down
+    // or stalls (give_up)
+    bool converged = h.done == 1, failed = h.done == 2 && h.nonfinite, give_up = false;
+    double rn_upd = h.rn;
+    int base = h.iters;
+    for (long long guard = 0; !converged && !failed && guard < ko.max_chunks; ++guard) {
+        if (!h.done) {
+            for (int k = 0; k < ko.chunk; ++k) iteration_mg(E, Af, V, cut);
+            LSMPS_CHECK_LAUNCH();
+            read();
         }
-        cudaGraphExec_t exec = nullptr;
-        if (o->use_graph == 2) {
-            cudaGraph_t graph;
-            LSMPS_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-            for (int c = 0; c < chunk; ++c) iteration<double, float>(E, Af, V, mgp);
-            note_launches(0 - kpi * (uint64_t)chunk);  // captured, not launched
-            cudaError_t e = cudaStreamEndCapture(s, &graph);
-            LSMPS_CUDA(e);
-            LSMPS_CUDA(cudaGraphInstantiate(&exec, graph, 0));
-            cudaGraphDestroy(graph);
+        total += h.iters - base;
+        base = h.iters;
+        if (!h.done && h.rn > ko.delta * rn_upd) continue;
+        const int why = h.done;  // 0: drop by delta; else the iteration stopped
+        if (why == 3 || total >= o->max_iter) {
+            // iteration cap: report the true residual of the last iterate
+            launch_replace(s, As, b, V, E);
+            read();
+            converged = h.done == 1;
+            break;
         }
-        bool give_up = false;
-        int base = h.iters;
-        for (long long guard = 0; !converged && !failed && guard < max_chunks; ++guard) {
-            if (!h.done) {
-                if (exec) {
-                    LSMPS_CUDA(cudaGraphLaunch(exec, s));
-                    note_launches(kpi * (uint64_t)chunk);
-                } else {
-                    for (int k = 0; k < chunk; ++k) iteration<double, float>(E, Af, V, mgp);
-                    LSMPS_CHECK_LAUNCH();
-                }
-                read(h);
-            }
-            total += h.iters - base;
-            base = h.iters;
-            if (!h.done && h.rn > delta * rn_upd) continue;
-            const int why = h.done;  // 0: drop by delta; else the iteration stopped
-            if (why == 3 || total >= o->max_iter) {
-                // iteration cap: report the true residual of the last iterate
-                launch_replace(s, As, b, V, E, nullptr, 0);
-                LSMPS_CHECK_LAUNCH();
-                read(h);
-                converged = h.done == 1;
-                break;
-            }
-            if (why == 0) {
-                launch_replace(s, As, b, V, E, nullptr, 0);
-                LSMPS_CHECK_LAUNCH();
-                ++replacements;
-                read(h);
-                rn_upd = h.rn;
-                if (h.done == 1) { converged = true; break; }
-                if (h.done == 0) continue;
-                // rho breakdown after the replacement: fall through to a restart
-            }
-            if (mgp && (h.done == 2 || h.done == 4)) { give_up = true; break; }
-            if (why == 4 && use_nn) fallback = 1;
-            if (h.nonfinite) { failed = true; break; }
-            // restart from the current iterate with the FP64 matrix (true residual)
-            set_scalar_caps(E, o->max_iter - total, restart_stall);
-            init<double, double>(E, As, b, V, true, o->tol, -1.0);
-            ++restarts;
-            read(h);
-            base = 0;
+        if (why == 0) {
+            launch_replace(s, As, b, V, E);
+            ++replacements;
+            read();
             rn_upd = h.rn;
             if (h.done == 1) { converged = true; break; }
-            if (h.done) { failed = true; break; }
+            if (h.done == 0) continue;
+            // rho breakdown after the replacement: fall through
         }
-        if (exec) cudaGraphExecDestroy(exec);
-        return give_up;
-    };
-    if (phase(mg)) {
+        if (h.done == 2 || h.done == 4) { give_up = true; break; }
+        if (h.nonfinite) { failed = true; break; }
+        // restart from the current iterate with the FP64 matrix (true residual)
+        set_scalar_caps(E, o->max_iter - total, stall);
+        init<double, double>(E, As, b, V, true, o->tol, -1.0);
+        ++restarts;
+        read();
+        base = 0;
+        rn_upd = h.rn;
+        if (h.done == 1) { converged = true; break; }
+        if (h.done) { failed = true; break; }
+    }
+    if (give_up) {
         // The multigrid broke down or stalled (near-singular aggregates can do this): continue
         // as Jacobi MIXED from the current iterate, or from zero if it is no longer finite.
-        fallback = 1;
-        const bool keep_x = !h.nonfinite;
-        if (!keep_x) LSMPS_CUDA(cudaMemsetAsync(V.x, 0, U * sizeof(double), s));
-        set_scalar_caps(E, o->max_iter - total, 0);
-        init<double, double>(E, As, b, V, keep_x, o->tol, -1.0);
-        ++restarts;
-        read(h);
-        converged = h.done == 1;
-        failed = h.done == 2;
-        if (total < o->max_iter) phase(false);
+        ko.use_nn = 0;
+        ko.warm_rn2 = nullptr;
+        ko.use_x = !h.nonfinite;
+        ko.max_iter = o->max_iter - total;
+        KrylovResult k = krylov_solve(ctx, &Af, As, K, ko);
+        k.iterations += total;
+        k.outer += replacements + restarts + 1;
+        k.fallback = 1;
+        return finish(k);
     }
     k_unscale<<<1184, 256, 0, s>>>(U, V.x, dinv);
     LSMPS_CHECK_LAUNCH();
     ev_record(ctx, 11);
-    LSMPS_CUDA(cudaStreamSynchronize(s));
     ps->iterations = total;
     ps->outer_iterations = replacements + restarts;
     ps->converged = converged;
     ps->fallback = fallback;
     ps->solve_ms = ev_elapsed(ctx, 10, 11);
-    if (exit_res) {
-        // convergence is only declared right after a residual replacement or a (re)start (in
-        // the device-driven loop too, which runs the same kernels in the same order), whose
-        // FP64 residual b - A D^-1 y of the final iterate h holds
-        const bool exact = converged && std::isfinite(h.rn);
-        exit_res[0] = exact ? h.rn : -1.0;
-        exit_res[1] = exact ? h.bnorm : -1.0;
+    if (converged && std::isfinite(h.rn)) {
+        exit_res[0] = h.rn;
+        exit_res[1] = h.bnorm;
     }
+    return false;
 }
 
 void ppe_set_initial_particles(lsmps_ctx* ctx, const double* pp, size_t n, bool device) {
@@ -1841,7 +1449,7 @@ void ppe_set_initial_particles(lsmps_ctx* ctx, const double* pp, size_t n, bool 
     LSMPS_REQUIRE(n == ctx->n && (n == 0 || pp), LSMPS_ERR_ARG, "initial guess must hold one value per particle");
     cudaStream_t s = ctx->stream;
     const long long U = ctx->U;
-    double* x = ctx->vx.ensure<double>(U + 1);
+    double* x = ctx->vx.ensure<double>(U + 2);
     const double* src = pp;
     if (!device && n) {
         double* tmp = ctx->vtmp.ensure<double>(n + 1);
@@ -1903,36 +1511,43 @@ void ppe_solve(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_stats* out)
         solve_exact(ctx, o, &ps);
     } else {
         double exit_res[2] = {-1.0, -1.0};
+        bool have_error = true;
         if (o->solver == LSMPS_SOLVER_FP64) solve_fast64(ctx, o, &ps, false);
         else if (o->solver == LSMPS_SOLVER_JACOBI) solve_fast64(ctx, o, &ps, true);
-        else if (o->solver == LSMPS_SOLVER_MIXED_F32) solve_mixed_f32(ctx, o, &ps, false);
-        else solve_mixed(ctx, o, &ps, o->solver == LSMPS_SOLVER_LEARNED, exit_res);
+        else if (o->solver == LSMPS_SOLVER_MIXED_F32) solve_mixed_f32(ctx, o, &ps, have_error = false);
+        else have_error = solve_mixed(ctx, o, &ps, o->solver == LSMPS_SOLVER_LEARNED, exit_res);
         // final statistics in FP64: |Ax - b|, |b| (for a converged MIXED / LEARNED solve the
         // convergence test's own FP64 residual of the final iterate, |b - A D^-1 y| with
-        // y = D x), error against p*
-        cudaStream_t s = ctx->stream;
-        Engine E = make_engine(ctx);
-        double* scal = engine_scalars(ctx);
-        double* x = ctx->vx.get<double>();
-        double* tmp = ctx->vt.ensure<double>(U + 1);
-        if (exit_res[0] < 0) residual64(E, sell_a64(ctx), ctx->A_b.get<double>(), x, tmp, scal);
-        auto* maxbits = reinterpret_cast<unsigned long long*>(scal + 4);
-        LSMPS_CUDA(cudaMemsetAsync(maxbits, 0, sizeof(unsigned long long), s));
-        k_error_stats<<<RGRID, RB, 0, s>>>(U, x, ctx->A_xexact.get<double>(), scal + 2, E.P, &E.S->counter[6],
-                                            maxbits);
-        LSMPS_CHECK_LAUNCH();
-        double h[5];
-        LSMPS_CUDA(cudaMemcpyAsync(h, scal, sizeof(h), cudaMemcpyDeviceToHost, s));
-        LSMPS_CUDA(cudaStreamSynchronize(s));
-        ps.initial_residual = exit_res[0] < 0 ? std::sqrt(h[1]) : exit_res[1];
-        ps.final_residual = exit_res[0] < 0 ? std::sqrt(h[0]) : exit_res[0];
+        // y = D x), error against p* (krylov.cu's solves bring their own)
+        if (exit_res[0] < 0 || !have_error) {
+            cudaStream_t s = ctx->stream;
+            Engine E = make_engine(ctx);
+            double* scal = engine_scalars(ctx);
+            double* x = ctx->vx.get<double>();
+            double* tmp = ctx->vt.ensure<double>(U + 2);
+            auto* maxbits = reinterpret_cast<unsigned long long*>(scal + 4);
+            set_scalar_caps(E, 0, 0);  // zeroes the reduction tickets
+            if (exit_res[0] < 0) residual64(E, sell_a64(ctx), ctx->A_b.get<double>(), x, tmp, scal);
+            LSMPS_CUDA(cudaMemsetAsync(maxbits, 0, sizeof(unsigned long long), s));
+            if (!have_error) {
+                k_error_stats<<<RGRID, RB, 0, s>>>(U, x, ctx->A_xexact.get<double>(), scal + 2, E.P, &E.S->counter[6],
+                                                    maxbits);
+                LSMPS_CHECK_LAUNCH();
+            }
+            double h[5];
+            read_back(ctx, {{scal, h, sizeof(h)}}, nullptr);
+            if (exit_res[0] < 0) {
+                exit_res[0] = std::sqrt(h[0]);
+                exit_res[1] = std::sqrt(h[1]);
+            }
+            if (!have_error) {
+                ps.relative_l2_error = std::sqrt(h[2] / std::max(h[3], 1e-30));
+                std::memcpy(&ps.max_error, &h[4], sizeof(double));
+            }
+        }
+        ps.initial_residual = exit_res[1];
+        ps.final_residual = exit_res[0];
         ps.relative_residual = ps.final_residual / std::max(ps.initial_residual, 1e-300);
-        ps.relative_l2_error = std::sqrt(h[2] / std::max(h[3], 1e-30));
-        unsigned long long mb;
-        std::memcpy(&mb, &h[4], sizeof(mb));
-        double mx;
-        std::memcpy(&mx, &mb, sizeof(mx));
-        ps.max_error = mx;
         if (!std::isfinite(ps.final_residual)) ps.converged = 0;
     }
     ctx->have_solution = true;
@@ -1946,13 +1561,7 @@ void solver_kernel_bench(lsmps_ctx* ctx, int kernel, int reps, double* ms, doubl
     LSMPS_REQUIRE(ctx->have_ppe, LSMPS_ERR_STATE, "SpMV bench needs an assembled PPE");
     cudaStream_t s = ctx->stream;
     const long long U = ctx->U;
-    Engine E = make_engine(ctx);
-    BcgScalars init{};
-    init.max_iter = 1 << 30;
-    init.rho = 1.0;
-    LSMPS_CUDA(cudaMemcpyAsync(E.S, &init, sizeof(init), cudaMemcpyHostToDevice, s));
     const bool f32 = kernel == LSMPS_KB_SPMV32;
-    // operands of ones: the fused dot is then nonzero, so no breakdown guard stops the kernel
     double* x = ctx->vp.ensure<double>(U + 1);
     double* r0 = ctx->vr0.ensure<double>(U + 1);
     double* y = ctx->vv.ensure<double>(U + 1);
@@ -1963,12 +1572,10 @@ void solver_kernel_bench(lsmps_ctx* ctx, int kernel, int reps, double* ms, doubl
     Sell<double> Ad{};
     if (f32) Af = sell_scaled32(ctx);
     else Ad = sell_a64(ctx);
+    const int* cut = f32 ? sell_cuts(ctx, Af) : sell_cuts(ctx, Ad);
     auto launch = [&] {
-        if (f32 && Af.dcol) k_bcg_v<double, float, true><<<spmv_grid<float, true>(), RB, 0, s>>>(Af, x, y, r0, E.S, E.P);
-        else if (f32) k_bcg_v<double, float, false><<<RGRID, RB, 0, s>>>(Af, x, y, r0, E.S, E.P);
-        else if (Ad.dcol) k_bcg_v<double, double, true><<<RGRID, RB, 0, s>>>(Ad, x, y, r0, E.S, E.P);
-        else k_bcg_v<double, double, false><<<RGRID, RB, 0, s>>>(Ad, x, y, r0, E.S, E.P);
-        LSMPS_CHECK_LAUNCH();
+        if (f32) krylov_row_product(ctx, Af, cut, x, y, r0);
+        else krylov_row_product(ctx, Ad, cut, x, y, r0);
     };
     launch();
     ev_record(ctx, 14);
