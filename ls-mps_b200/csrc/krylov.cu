@@ -7,11 +7,11 @@
 // residual replacement, restart, fallback) for itself, from the same bits. So an iteration has
 // no launches, no last-block serial step and no host round trip.
 //
-// What bounds it: the row products' matrix stream for large systems (2 x 40 us of a 911k-unknown
-// iteration's 100), their gathers' latency at ~200k (2 x 13 of 37 us), and for small systems the
+// What bounds it: the row products' matrix stream for large systems (2 x 41 us of a 911k-unknown
+// iteration's 102), their gathers' latency at ~180k (2 x 13 of 38 us), and for small systems the
 // barriers: 1.5 us each, 2.4 us with sums, five per iteration. As five kernels per iteration with a
-// last-block sum in each an iteration took 31 us at 6,000 unknowns (17 now), 49 us at 181k (37)
-// and 108 us at 911k (100).
+// last-block sum in each, host-launched, an iteration took 35.0 us at 6,000 unknowns (17.5 now),
+// 52 us at 181k (37.9) and 117 us at 911k (102).
 //
 // Waits are bounded: a block that polls a barrier longer than SPIN_LIMIT times raises
 // DFLAG_TIMEOUT and ends, and so does every block after it.

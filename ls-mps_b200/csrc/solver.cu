@@ -42,9 +42,8 @@ struct Partials {
 
 // Block sum of two doubles into partials[blockIdx]; returns true in the last block to
 // arrive, after which the caller may read all partials (fixed-order final sum).
-template <int NT = RB>
 __device__ __forceinline__ bool block_partials(double va, double vb, Partials P, unsigned int* counter) {
-    __shared__ double sa[NT / 32], sb[NT / 32];
+    __shared__ double sa[RB / 32], sb[RB / 32];
     __shared__ bool last;
     va = warp_sum(va);
     vb = warp_sum(vb);
@@ -53,7 +52,7 @@ __device__ __forceinline__ bool block_partials(double va, double vb, Partials P,
     __syncthreads();
     if (threadIdx.x == 0) {
         double ta = 0, tb = 0;
-        for (int k = 0; k < NT / 32; ++k) { ta += sa[k]; tb += sb[k]; }
+        for (int k = 0; k < RB / 32; ++k) { ta += sa[k]; tb += sb[k]; }
         P.a[blockIdx.x] = ta;
         P.b[blockIdx.x] = tb;
         __threadfence();
@@ -64,13 +63,12 @@ __device__ __forceinline__ bool block_partials(double va, double vb, Partials P,
     return last;
 }
 
-// In the last block: fixed-order sum of the partials (thread t sums entries t, t+NT, ...
+// In the last block: fixed-order sum of the partials (thread t sums entries t, t+RB, ...
 // then a fixed tree), result in *ra / *rb for thread 0.
-template <int NT = RB>
 __device__ __forceinline__ void final_sum(Partials P, double* ra, double* rb) {
-    __shared__ double sa[NT / 32], sb[NT / 32];
+    __shared__ double sa[RB / 32], sb[RB / 32];
     double va = 0, vb = 0;
-    for (int k = threadIdx.x; k < (int)gridDim.x; k += NT) {
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += RB) {
         va += __ldcg(P.a + k);
         vb += __ldcg(P.b + k);
     }
@@ -80,7 +78,7 @@ __device__ __forceinline__ void final_sum(Partials P, double* ra, double* rb) {
     __syncthreads();
     if (threadIdx.x == 0) {
         double ta = 0, tb = 0;
-        for (int k = 0; k < NT / 32; ++k) { ta += sa[k]; tb += sb[k]; }
+        for (int k = 0; k < RB / 32; ++k) { ta += sa[k]; tb += sb[k]; }
         *ra = ta;
         *rb = tb;
     }
@@ -311,10 +309,10 @@ __global__ void __launch_bounds__(RB) k_bcg_s_agg(MgFine G, const double* __rest
     }
 }
 
-// t = A s; omega = (t, s) / (t, t)
+// t = A s; omega = (t, s) / (t, t). sd: the s of the dot where sv is a preconditioned M s.
 template <class T, class TM = T, bool C16 = false>
 __global__ void __launch_bounds__(RB, spmv_blocks_per_sm<TM, C16>()) k_bcg_t(Sell<TM> A, const T* __restrict__ sv, T* __restrict__ t,
-                                              BcgScalars* S, Partials P) {
+                                              BcgScalars* S, Partials P, const T* __restrict__ sd) {
     pdl_begin();
     if (S->done || S->s_conv) return;
     double ats = 0, att = 0;
@@ -324,76 +322,13 @@ __global__ void __launch_bounds__(RB, spmv_blocks_per_sm<TM, C16>()) k_bcg_t(Sel
         if (i < A.n) {
             T ti = (T)y;
             t[i] = ti;
-            ats += (double)ti * (double)sv[i];
+            ats += (double)ti * (double)sd[i];
             att += (double)ti * (double)ti;
         }
     }
     if (block_partials(ats, att, P, &S->counter[2])) {
         double ts, tt;
         final_sum(P, &ts, &tt);
-        if (threadIdx.x == 0) {
-            S->counter[2] = 0;
-            S->tt = tt;
-            if (!isfinite(tt) || !isfinite(ts)) { S->nonfinite = 1; S->done = 2; }
-            else if (tt < 1e-30) S->done = 2;
-            else S->omega = ts / tt;
-        }
-    }
-}
-
-// The row products of the multigrid's iteration: one block of 1,024 threads per SM over a
-// contiguous run of slices (cut[b] .. cut[b + 1], about the same stored entries each), so that an
-// SM's gathers share lines in its L1. sd: t = A sv with the preconditioned sv = M s, whose dot takes s itself.
-constexpr int MGT = 1024;
-template <bool C16>
-__global__ void __launch_bounds__(MGT, 1) k_mg_v(Sell<float> A, const int* __restrict__ cut, const double* __restrict__ p,
-                                                 double* __restrict__ v, const double* __restrict__ r0, BcgScalars* S,
-                                                 Partials P) {
-    const int lane = threadIdx.x & 31, s1 = cut[blockIdx.x + 1];
-    int s = cut[blockIdx.x] + (threadIdx.x >> 5);  // (written before the solve)
-    pdl_begin();
-    if (S->done) return;
-    double acc = 0;
-    for (; s < s1; s += MGT / 32) {
-        const double y = sell_product<C16>(A, s, lane, p);
-        const long long i = ((long long)s << 5) + lane;
-        if (i < A.n) {
-            v[i] = y;
-            acc += r0[i] * y;
-        }
-    }
-    if (block_partials<MGT>(acc, 0.0, P, &S->counter[0])) {
-        double den, unused;
-        final_sum<MGT>(P, &den, &unused);
-        if (threadIdx.x == 0) {
-            S->counter[0] = 0;
-            if (!isfinite(den)) { S->nonfinite = 1; S->done = 2; }
-            else if (fabs(den) < 1e-30) S->done = 2;
-            else S->alpha = S->rho / den;
-        }
-    }
-}
-template <bool C16>
-__global__ void __launch_bounds__(MGT, 1) k_mg_t(Sell<float> A, const int* __restrict__ cut, const double* __restrict__ sv,
-                                                 double* __restrict__ t, const double* __restrict__ sd, BcgScalars* S,
-                                                 Partials P) {
-    const int lane = threadIdx.x & 31, s1 = cut[blockIdx.x + 1];
-    int s = cut[blockIdx.x] + (threadIdx.x >> 5);
-    pdl_begin();
-    if (S->done || S->s_conv) return;
-    double ats = 0, att = 0;
-    for (; s < s1; s += MGT / 32) {
-        const double y = sell_product<C16>(A, s, lane, sv);
-        const long long i = ((long long)s << 5) + lane;
-        if (i < A.n) {
-            t[i] = y;
-            ats += y * sd[i];
-            att += y * y;
-        }
-    }
-    if (block_partials<MGT>(ats, att, P, &S->counter[2])) {
-        double ts, tt;
-        final_sum<MGT>(P, &ts, &tt);
         if (threadIdx.x == 0) {
             S->counter[2] = 0;
             S->tt = tt;
@@ -898,25 +833,25 @@ void iteration(Engine& E, const Sell<T>& A, const Vecs<T>& V) {
     if (A.dcol) launch_pdl(k_bcg_v<T, T, true>, spmv_grid<T, true>(), RB, 0, E.s, A, V.p, V.v, V.r0, E.S, E.P);
     else launch_pdl(k_bcg_v<T, T, false>, RGRID, RB, 0, E.s, A, V.p, V.v, V.r0, E.S, E.P);
     launch_pdl(k_bcg_s<T>, RGRID, RB, 0, E.s, A.n, V.r, V.v, V.s, E.S, E.P);
-    if (A.dcol) launch_pdl(k_bcg_t<T, T, true>, spmv_grid<T, true>(), RB, 0, E.s, A, V.s, V.t, E.S, E.P);
-    else launch_pdl(k_bcg_t<T, T, false>, RGRID, RB, 0, E.s, A, V.s, V.t, E.S, E.P);
+    if (A.dcol) launch_pdl(k_bcg_t<T, T, true>, spmv_grid<T, true>(), RB, 0, E.s, A, V.s, V.t, E.S, E.P, V.s);
+    else launch_pdl(k_bcg_t<T, T, false>, RGRID, RB, 0, E.s, A, V.s, V.t, E.S, E.P, V.s);
     launch_pdl(k_bcg_x<T, false>, RGRID, RB, 0, E.s, A.n, V.x, V.r, V.p, V.s, V.t, V.r0, E.S, E.P, (const T*)nullptr,
                (const T*)nullptr);
 }
 
 // One iteration with the multigrid V-cycle as the right preconditioner: p (and s) and its
 // level-1 restriction in one pass, the rest of the V-cycle, then the row product.
-void iteration_mg(Engine& E, const Sell<float>& A, const Vecs<double>& V, const int* cut) {
+void iteration_mg(Engine& E, const Sell<float>& A, const Vecs<double>& V) {
     note_launches(5);
     const MgFine G = mg_fine(E.ctx);
     launch_pdl(k_bcg_p_agg, agg_blocks(G.n1), RB, 0, E.s, G, V.r, V.p, V.v, E.S);
     mg_apply(E.ctx, V.p, V.ph, E.S, 0, true);
-    if (A.dcol) launch_pdl(k_mg_v<true>, SELL_CUTS, MGT, 0, E.s, A, cut, V.ph, V.v, V.r0, E.S, E.P);
-    else launch_pdl(k_mg_v<false>, SELL_CUTS, MGT, 0, E.s, A, cut, V.ph, V.v, V.r0, E.S, E.P);
+    if (A.dcol) launch_pdl(k_bcg_v<double, float, true>, spmv_grid<float, true>(), RB, 0, E.s, A, V.ph, V.v, V.r0, E.S, E.P);
+    else launch_pdl(k_bcg_v<double, float, false>, RGRID, RB, 0, E.s, A, V.ph, V.v, V.r0, E.S, E.P);
     launch_pdl(k_bcg_s_agg, std::min<unsigned>(RGRID, agg_blocks(G.n1)), RB, 0, E.s, G, V.r, V.v, V.s, E.S, E.P);
     mg_apply(E.ctx, V.s, V.sh, E.S, 1, true);
-    if (A.dcol) launch_pdl(k_mg_t<true>, SELL_CUTS, MGT, 0, E.s, A, cut, V.sh, V.t, V.s, E.S, E.P);
-    else launch_pdl(k_mg_t<false>, SELL_CUTS, MGT, 0, E.s, A, cut, V.sh, V.t, V.s, E.S, E.P);
+    if (A.dcol) launch_pdl(k_bcg_t<double, float, true>, spmv_grid<float, true>(), RB, 0, E.s, A, V.sh, V.t, E.S, E.P, V.s);
+    else launch_pdl(k_bcg_t<double, float, false>, RGRID, RB, 0, E.s, A, V.sh, V.t, E.S, E.P, V.s);
     launch_pdl(k_bcg_x<double, true>, RGRID, RB, 0, E.s, A.n, V.x, V.r, V.p, V.s, V.t, V.r0, E.S, E.P, V.ph, V.sh);
 }
 
@@ -1354,7 +1289,6 @@ static bool solve_mixed(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_st
         W.keep = V.s;
         return finish(krylov_solve(ctx, &Af, As, W, ko));
     }
-    const int* cut = sell_cuts(ctx, Af);
     set_scalar_caps(E, o->max_iter, stall);
     if (!ko.use_x) LSMPS_CUDA(cudaMemsetAsync(V.x, 0, U * sizeof(double), s));
     init<double, double>(E, As, b, V, ko.use_x != 0, o->tol, -1.0);
@@ -1379,7 +1313,7 @@ static bool solve_mixed(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_st
     int base = h.iters;
     for (long long guard = 0; !converged && !failed && guard < ko.max_chunks; ++guard) {
         if (!h.done) {
-            for (int k = 0; k < ko.chunk; ++k) iteration_mg(E, Af, V, cut);
+            for (int k = 0; k < ko.chunk; ++k) iteration_mg(E, Af, V);
             LSMPS_CHECK_LAUNCH();
             read();
         }
