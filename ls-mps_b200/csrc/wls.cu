@@ -260,6 +260,10 @@ struct WlsParams {
     double coef[30];  // nrhs x 10
 };
 
+__device__ __forceinline__ double quad_fast(const double* c, double x, double y, double z) {
+    return c[0] + c[1] * x + c[2] * y + c[3] * z + c[4] * x * x + c[5] * y * y + c[6] * z * z + c[7] * x * y +
+           c[8] * x * z + c[9] * y * z;
+}
 // gradient of the quadratic field c at (x, y, z)
 __device__ __forceinline__ void quad_grad(const double* c, double x, double y, double z, double* g) {
     g[0] = c[1] + 2 * c[4] * x + c[7] * y + c[8] * z;
@@ -349,7 +353,7 @@ __device__ __forceinline__ double accumulate_moments(int k, const double* __rest
 // One pass over the neighbors for both the moments (as accumulate_moments) and the
 // right-hand sides B[f]_a = sum w q_a (f_m - f_k) / r = c_a sum W (f_m - f_k) mono_a, in the
 // neighbor order. Returns sum w.
-template <int NRHS>
+template <int NRHS, bool ARRAY>
 __device__ __forceinline__ double accumulate_moments_rhs(int k, const double* __restrict__ sx,
                                                          const double* __restrict__ sy,
                                                          const double* __restrict__ sz,
@@ -366,12 +370,14 @@ __device__ __forceinline__ double accumulate_moments_rhs(int k, const double* __
         for (int a = 0; a < K; ++a) B[f][a] = 0;
     const double xi = sx[k], yi = sy[k], zi = sz[k];
     double ws = 0;
-    double fi[NRHS], gf[NRHS][3];  // the field's value at k (array), or its gradient there
+    // field values: per-particle array (sorted order, NRHS per particle) or the analytic
+    // quadratics. (The quadratics' differences are taken of their values, as the array's are:
+    // formed from the gradient at k they are rounded differently, which the nearly singular
+    // systems show at 1e-7 of the solution.)
+    double fi[NRHS];
 #pragma unroll
-    for (int f = 0; f < NRHS; ++f) {
-        fi[f] = fvals ? fvals[(size_t)k * NRHS + f] : 0.0;
-        quad_grad(P.coef + 10 * f, xi, yi, zi, gf[f]);
-    }
+    for (int f = 0; f < NRHS; ++f)
+        fi[f] = ARRAY ? fvals[(size_t)k * NRHS + f] : quad_fast(P.coef + 10 * f, xi, yi, zi);
     // the next neighbor's position (and the index after it) are loaded while this one's terms
     // are summed
     const int e1 = row[k + 1];
@@ -397,12 +403,8 @@ __device__ __forceinline__ double accumulate_moments_rhs(int k, const double* __
         if (P.mirror_walls && cls[mc] == LSMPS_WALL) continue;  // f_m = f_k: no right-hand-side term
 #pragma unroll
         for (int f = 0; f < NRHS; ++f) {
-            // f_m - f_k; of a quadratic field from its gradient at k and its second derivatives
-            const double* c = P.coef + 10 * f;
-            const double df = fvals ? fvals[(size_t)mc * NRHS + f] - fi[f]
-                                    : gf[f][0] * dx + gf[f][1] * dy + gf[f][2] * dz + c[4] * p[0] + c[5] * p[3] +
-                                          c[6] * p[5] + c[7] * p[1] + c[8] * p[2] + c[9] * p[4];
-            const double g = df * W;
+            const double fm = ARRAY ? fvals[(size_t)mc * NRHS + f] : quad_fast(P.coef + 10 * f, xc, yc, zc);
+            const double g = (fm - fi[f]) * W;
             B[f][0] += g * dx, B[f][1] += g * dy, B[f][2] += g * dz;
             B[f][3] += g * p[0], B[f][4] += g * p[3], B[f][5] += g * p[5];
             B[f][6] += g * p[1], B[f][7] += g * p[2], B[f][8] += g * p[4];
@@ -468,24 +470,25 @@ __device__ void atomic_max_nonneg(double* addr, double v) {
 
 // The right-hand sides accumulate in the moments' neighbor pass (one pass over the neighbors;
 // measured 22 % faster at 1M particles than a second right-hand-side pass, for 2 more registers).
-// Bound by the FP64 pipe's latency at 12 warps per SM. At 1M particles one field takes 313 us
-// (443 before the neighbor loop loaded one neighbor ahead and took an analytic field's
-// differences from its gradient at k), three caller fields 511 us (874, and 386 more for the copy
-// of the solutions to the caller's order, where they are now written directly).
+// Bound by the FP64 pipe's latency at 12 warps per SM. At 1M particles one analytic field takes
+// 307 us (454 before the neighbor loop loaded one neighbor ahead and blocks were one warp), three
+// caller fields (ARRAY) 524 us (774, and 386 more for the copy of the solutions to the caller's
+// order, where they are now written directly).
 // One warp per block, so a warp's registers are free for the next one as soon as it ends (rows
 // of uneven length): blocks of 64 and 128 threads took 5 and 17 % longer.
-// Registers: one FP64 field takes 166 by itself, 12 warps per SM. Two and three fields would take
-// 192-216 (8-10 warps) and are capped at 168: 464 against 597 us (two) and 651 against 649
-// (three) at 1M, 32 against 46 and 42 against 50 at 50k. Mixed precision with one field is capped
-// too (499 against 562 us at 1M), with more the spills cost more than the warps gain (three
-// fields at 100k: 139 capped against 113).
-template <int NRHS, int PREC>
+// Registers, us at 1M capped at 168 (12 warps per SM) against uncapped (192-216 registers, 8-10
+// warps): FP64 two fields 389 against 444, two caller fields 422 against 523, three caller fields
+// 524 against 578 are capped; three analytic fields 523 against 516 (100k: 71 against 63) and one
+// field (164 registers by itself, 320 against 309) are not. Mixed precision with one field is
+// capped (475 against 502), with two and three the spills cost more than the warps gain (702
+// against 638, 1000 against 813).
+template <int NRHS, int PREC, bool ARRAY>
 constexpr int wls_regs() {
-    return (NRHS == 1) == (PREC == 0) ? 255 : 168;
+    return (PREC ? NRHS == 1 : NRHS == 2 || (NRHS == 3 && ARRAY)) ? 168 : 255;
 }
 constexpr int WLS_SLOTS = 16;  // copies of the statistics, so that the blocks' atomics spread
-template <int NRHS, int PREC>
-__global__ void __maxnreg__((wls_regs<NRHS, PREC>())) k_wls_all(WlsParams P, int n, const uint8_t* __restrict__ cls,
+template <int NRHS, int PREC, bool ARRAY>
+__global__ void __maxnreg__((wls_regs<NRHS, PREC, ARRAY>())) k_wls_all(WlsParams P, int n, const uint8_t* __restrict__ cls,
                                                  const double* __restrict__ sx, const double* __restrict__ sy,
                                                  const double* __restrict__ sz, const int* __restrict__ row,
                                                  const int* __restrict__ col, int* __restrict__ status,
@@ -509,7 +512,7 @@ __global__ void __maxnreg__((wls_regs<NRHS, PREC>())) k_wls_all(WlsParams P, int
             const double xi = sx[k], yi = sy[k], zi = sz[k];
             // right-hand sides: the quadratic fields (the Laplacian vector is solved separately)
             double B[NRHS][K];
-            double ws = accumulate_moments_rhs<NRHS>(k, sx, sy, sz, row, col, cls, P, l0inv, fvals, L, B);
+            double ws = accumulate_moments_rhs<NRHS, ARRAY>(k, sx, sy, sz, row, col, cls, P, l0inv, fvals, L, B);
             wsum[k] = ws;
             if (!(ws > 0)) {
                 my_status = W_NOWEIGHT;
@@ -612,7 +615,7 @@ __global__ void __maxnreg__((wls_regs<NRHS, PREC>())) k_wls_all(WlsParams P, int
 #pragma unroll
                             for (int a = 0; a < K; ++a) xout[o + a] = B[f][a];
                         }
-                        if (fvals) continue;  // no analytic field to measure against
+                        if (ARRAY) continue;  // no analytic field to measure against
                         const double* c = P.coef + 10 * f;
                         double gr[3];
                         quad_grad(c, xi, yi, zi, gr);
@@ -663,7 +666,7 @@ struct WlsOut {
     const int* xperm = nullptr;
 };
 
-template <int NRHS, int PREC>
+template <int NRHS, int PREC, bool ARRAY = false>
 void launch_all(lsmps_ctx* ctx, const WlsParams& P, unsigned long long* gcnt,
                 const double* fvals = nullptr, const WlsOut* dst = nullptr) {
     int n = (int)ctx->n;
@@ -671,7 +674,7 @@ void launch_all(lsmps_ctx* ctx, const WlsParams& P, unsigned long long* gcnt,
     const WlsOut o = dst ? *dst
                          : WlsOut{ctx->wls_status.get<int>(), ctx->wls_z.get<double>(), ctx->wls_wsum.get<double>(),
                                   ctx->wls_x.get<double>()};
-    k_wls_all<NRHS, PREC><<<blocks_for(n, 32), 32, 0, ctx->stream>>>(
+    k_wls_all<NRHS, PREC, ARRAY><<<blocks_for(n, 32), 32, 0, ctx->stream>>>(
         P, n, ctx->cls.get<uint8_t>(), ctx->sx.get<double>(), ctx->sy.get<double>(), ctx->sz.get<double>(),
         ctx->nbr_row.get<int>(), ctx->nbr_col.get<int>(), o.status, o.z, o.wsum, o.x, gcnt, fvals, o.xperm);
     LSMPS_CHECK_LAUNCH();
@@ -827,9 +830,9 @@ void wls_fields(lsmps_ctx* ctx, const double* d_fields, int nrhs, double* d_out,
                                                                                       d_fields, fs);
         LSMPS_CHECK_LAUNCH();
     }
-    if (nrhs == 1) launch_all<1, 0>(ctx, P, gcnt, fs, &o);
-    else if (nrhs == 2) launch_all<2, 0>(ctx, P, gcnt, fs, &o);
-    else launch_all<3, 0>(ctx, P, gcnt, fs, &o);
+    if (nrhs == 1) launch_all<1, 0, true>(ctx, P, gcnt, fs, &o);
+    else if (nrhs == 2) launch_all<2, 0, true>(ctx, P, gcnt, fs, &o);
+    else launch_all<3, 0, true>(ctx, P, gcnt, fs, &o);
 }
 
 void wls_kernel_bench(lsmps_ctx* ctx, int reps, double* ms, double* bytes) {
