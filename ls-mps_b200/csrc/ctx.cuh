@@ -88,7 +88,7 @@ struct lsmps_ctx {
     int nsegs = 0;  // non-empty 12-cell segments of the grid (neighbor passes)
     lsmps_gpu::DevBuf cell_of, slot, cell_count, cell_start, perm, iperm;
     lsmps_gpu::DevBuf sx, sy, sz, stype, scell, cls;
-    lsmps_gpu::DevBuf nbr_cnt, nbr_row, nbr_col, nbr_stats, seg_list;
+    lsmps_gpu::DevBuf nbr_cnt, nbr_row, nbr_col, nbr_stats, seg_list, scan_items, scan_rel;
     lsmps_gpu::DevBuf nbr_slots;  // single-pass build: maxn slots per particle before compaction
     bool nbr_single = false;      // the last build used the single pass
     // candidate lists of radius re + skin (sorted numbering) and the sorted positions they

@@ -358,14 +358,18 @@ struct SegGrid {
     int nsegx;
 };
 
+// The decisions are safe when no component is within `margin` of zero and the largest is that far
+// above the other two.
 __device__ __forceinline__ bool sector_bits_f32(float dx, float dy, float dz, float margin, unsigned& bits) {
     const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
-    if (fminf(fminf(ax, ay), az) <= margin || fabsf(ax - ay) <= margin || fabsf(ax - az) <= margin ||
-        fabsf(ay - az) <= margin)
+    const float lo = fminf(ax, ay), hi = fmaxf(ax, ay), top = fmaxf(hi, az);
+    if (fminf(lo, az) <= margin || top - fmaxf(lo, fminf(hi, az)) <= margin) {
+        bits = 0;
         return false;
-    const int s = (ax >= ay && ax >= az) ? (dx >= 0 ? 0 : 1) : ((ay >= ax && ay >= az) ? (dy >= 0 ? 2 : 3) : (dz >= 0 ? 4 : 5));
-    const int o = 6 + (dx >= 0) + 2 * (dy >= 0) + 4 * (dz >= 0);
-    bits = (1u << s) | (1u << o);
+    }
+    const unsigned sx = __float_as_uint(dx) >> 31, sy = __float_as_uint(dy) >> 31, sz = __float_as_uint(dz) >> 31;
+    const unsigned s = az == top ? 4 + sz : (ay == top ? 2 + sy : sx);
+    bits = (1u << s) | ((1u << 13) >> (sx + 2 * sy + 4 * sz));
     return true;
 }
 
@@ -539,200 +543,257 @@ __global__ void __launch_bounds__(SEG_THREADS, 8) k_seg_pass(SegGrid G, const in
 }
 
 // ---- single pass: each query's kept list straight into its slot row ------------------------
-// The staging, the cell culling and the FP32 guard band of k_seg_pass, in one pass instead of
-// a count and a fill pass that repeat every distance test. A thread tests its row window 32
-// staged candidates at a time into a hit mask (no branch per candidate), then walks the set
-// bits in order: the rare guard-band hits are decided exactly in FP64, and each kept candidate
-// p < maxn goes to slots[k * maxn + p] with its sector bits. Counting continues past maxn for
-// the truncation statistic. k_slots_compact then packs the slot rows into the CSR once the
-// kept counts are scanned. The kept order is the staged order of the 9 row windows, which is
-// the reference's order, as in k_seg_pass.
-__device__ __forceinline__ void scan_query_global(const GridView& g, const double* __restrict__ sx,
-                                                  const double* __restrict__ sy, const double* __restrict__ sz,
-                                                  const int* __restrict__ scell, const uint8_t* __restrict__ stype,
-                                                  int k, double re2, int maxn, double l0, int classify,
-                                                  int* __restrict__ slots, int* __restrict__ cnt,
-                                                  unsigned long long* trunc_total, uint8_t* __restrict__ cls,
-                                                  int lane) {
-    const unsigned lt = (1u << lane) - 1u;
-    const int lin = scell[k];
-    const int cx = lin % g.nx, t = lin / g.nx, cy = t % g.ny, cz = t / g.ny;
-    const double xi = sx[k], yi = sy[k], zi = sz[k];
-    int* out = slots + (size_t)k * maxn;
-    int written = 0;
-    unsigned sec = 0;
-    for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy) {
-            int beg, end;
-            if (!row_range(g, cx, cy, cz, dy, dz, beg, end)) continue;
-            for (int mb = beg; mb < end; mb += 32) {
-                const int m = mb + lane;
-                bool ok = false;
-                double dx = 0, dyv = 0, dzv = 0;
-                if (m < end && m != k) {
-                    dx = xsub(sx[m], xi);
-                    dyv = xsub(sy[m], yi);
-                    dzv = xsub(sz[m], zi);
-                    ok = xnorm2(dx, dyv, dzv) < re2;
-                }
-                const unsigned bal = __ballot_sync(0xffffffffu, ok);
-                if (ok) {
-                    const int p = written + __popc(bal & lt);
-                    if (p < maxn) {
-                        out[p] = m;
-                        if (classify) sec |= sector_bits(dx, dyv, dzv);
-                    }
-                }
-                written += __popc(bal);
-            }
-        }
-    if (lane == 0) {
-        cnt[k] = min(written, maxn);
-        if (written > maxn) atomicAdd(trunc_total, (unsigned long long)(written - maxn));
+// One warp per cell and 32 of its particles (the queries). The cell's candidates, the particles
+// of its 27 cells in the reference's order (9 rows of three cells, contiguous in the sorted
+// order), go into registers, one per lane and chunk of 32, as FP32 positions relative to the
+// cell's corner. The warp then takes the queries one by one: every lane tests its candidates
+// with packed FP32x2 arithmetic, the ballots of a chunk are the hits in order, the hits are
+// packed into shared memory and from there, a lane each, written to slots[k * maxn + p] for
+// p < maxn, with their sector bits for the classification. A query with a candidate in the
+// guard band of k_seg_pass (|d^2 - re^2| <= 2.1e-5 re^2; the FP32 distance^2 is within 1e-6 re^2
+// of the exact one) has its hits there decided exactly in FP64, so the kept lists are the
+// reference's bit for bit. Cells of more than SCAN_CH chunks take them in turns. Counting
+// continues past maxn for the truncation statistic. k_slots_compact then packs the slot rows
+// into the CSR once the kept counts are scanned.
+// What bounds it: the latency of a query's chain (ballots, packing, sector bits) at 16 warps per
+// SM; two queries at a time hide half of it (one at a time took 518 us at 1M). It took the place
+// of a block per 12-cell segment with a thread per query, which was bound by shared memory (24
+// bytes per candidate pair and lane) and by the divergent walk over each thread's hits, with a
+// third to a half of the lanes idle: 532 us for 1M particles of a mixed set (479 now), 172 us for
+// 200k of a rain set (111) and 890 for 1M at radius 2.3 (513). Five blocks per SM (102
+// registers, spilled) took 499 us, three 565.
+constexpr int SCAN_CH = 10;     // chunks of 32 candidates in registers (a cell of side 2.1 has 250 candidates)
+constexpr int SCAN_WARPS = 4;   // per block
+
+// Items of the scan (cell x, y, z and first query), in any order (an item's outputs are addressed by its
+// own particles): items[0].x is their number, items[0].y how many the scan has drawn. rel: each particle's position relative to its
+// cell's corner, and the cell's x index.
+__global__ void k_scan_prep(GridView g, int3 g0, double re, long long ncells, int n, const int* __restrict__ scell,
+                            const double* __restrict__ sx, const double* __restrict__ sy,
+                            const double* __restrict__ sz, int4* __restrict__ items, float4* __restrict__ rel) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    int q0 = 0, blocks = 0;
+    if (t < ncells) {
+        q0 = g.cell_start[t];
+        blocks = (g.cell_start[t + 1] - q0 + 31) >> 5;
     }
-    if (classify) {
-        sec = __reduce_or_sync(0xffffffffu, sec);
-        if (lane == 0) cls[k] = classify_rule(stype[k], min(written, maxn), sec, zi, l0);
+    const int lane = threadIdx.x & 31;
+    int sum = blocks;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+    }
+    int base = 0;
+    if (lane == 31 && sum) base = atomicAdd(&items[0].x, sum);
+    base = __shfl_sync(0xffffffffu, base, 31) + sum - blocks + 1;
+    if (blocks) {
+        const int u = (int)t / g.nx;
+        for (int b = 0; b < blocks; ++b)
+            items[base + b] = make_int4((int)t % g.nx, u % g.ny, u / g.ny, q0 + 32 * b);
+    }
+    if (t < n) {
+        const int lin = scell[t], cx = lin % g.nx, u = lin / g.nx, cy = u % g.ny, cz = u / g.ny;
+        rel[t] = make_float4((float)(sx[t] - (g0.x + cx) * re), (float)(sy[t] - (g0.y + cy) * re),
+                             (float)(sz[t] - (g0.z + cz) * re), __int_as_float(cx));
     }
 }
 
-__global__ void __launch_bounds__(SEG_THREADS, 8) k_seg_scan(SegGrid G, const int* __restrict__ seg_list,
-                                                            const double* __restrict__ sx,
-                                                            const double* __restrict__ sy,
-                                                            const double* __restrict__ sz,
-                                                            const int* __restrict__ scell,
-                                                            const uint8_t* __restrict__ stype, double re2,
-                                                            int maxn, double l0, int classify,
-                                                            int* __restrict__ cnt,
-                                                            unsigned long long* trunc_total,
-                                                            int* __restrict__ slots, uint8_t* __restrict__ cls) {
-    // staged candidates in pairs, for the packed FP32x2 arithmetic: pair p holds the x and y
-    // of candidates 2p and 2p + 1 in cxy[p] and their z in cz[p]
-    __shared__ float4 cxy[SEG_MAXC / 2 + 1];
-    __shared__ float2 cz[SEG_MAXC / 2 + 1];
-    __shared__ int rbase[10], rfirst[9], rcs[9][SEG + 3];
-    const float re_f = (float)G.re;
+__global__ void __launch_bounds__(32 * SCAN_WARPS, 4) k_cell_scan(
+    GridView g, int n, int4* __restrict__ items, const float4* __restrict__ rel, const double* __restrict__ sx,
+    const double* __restrict__ sy, const double* __restrict__ sz, const uint8_t* __restrict__ stype, float re_f,
+    double re2, int maxn, double l0, int classify, int* __restrict__ cnt, unsigned long long* trunc_total,
+    int* __restrict__ slots, uint8_t* __restrict__ cls) {
+    __shared__ float4 packed[SCAN_WARPS][2 * 32 * SCAN_CH];  // two queries' hits: position and index
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    float4* hits = packed[warp];
     const float re2f = (float)re2;
-    const float lo_th = re2f * (1.f - 2e-5f), hi_th = re2f * (1.f + 2e-5f);
-    const float cull = re2f * (1.f + 1e-4f);
+    const float lo_th = re2f * (1.f - 2e-5f), hi_th = re2f * (1.f + 2e-5f), band = 2.1e-5f * re2f;
     const float margin = 4e-6f * re_f;
-    const int seg = seg_list[blockIdx.x];
-    const int sxi = seg % G.nsegx, tt = seg / G.nsegx, cy = tt % G.g.ny, cz0 = tt / G.g.ny;
-    const int cx0 = sxi * SEG, cx1 = min(cx0 + SEG, G.g.nx) - 1;
-    const int lo = max(cx0 - 1, 0), hi = min(cx1 + 1, G.g.nx - 1);
-    const int rowlin = (cz0 * G.g.ny + cy) * G.g.nx;
-    const int q0 = G.g.cell_start[rowlin + cx0], q1 = G.g.cell_start[rowlin + cx1 + 1];
-    for (int t = threadIdx.x; t < 9 * (SEG + 3); t += blockDim.x) {
-        const int r = t / (SEG + 3), c = lo + t % (SEG + 3);
-        const int y = cy + (r % 3 - 1), z = cz0 + (r / 3 - 1);
-        int v = 0;
-        if (y >= 0 && y < G.g.ny && z >= 0 && z < G.g.nz && c <= hi + 1) v = G.g.cell_start[(z * G.g.ny + y) * G.g.nx + c];
-        rcs[r][c - lo] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        rbase[0] = 0;
-        for (int r = 0; r < 9; ++r) {
-            rfirst[r] = rcs[r][0];
-            rbase[r + 1] = rbase[r] + (rcs[r][hi + 1 - lo] - rcs[r][0]);
+    const int nitems = items[0].x;
+    // An item's number, cell, row ranges and candidates are four dependent loads: the first three
+    // are made one to three items ahead. The first items go by the warp's number, the others are
+    // drawn from a counter.
+    const int first = blockIdx.x * SCAN_WARPS + warp;
+    int drawn = 0;  // in lane 0
+    auto draw = [&] {
+        if (lane == 0) drawn = gridDim.x * SCAN_WARPS + atomicAdd(&items[0].y, 1);
+    };
+    auto after = [&] {
+        const int it = __shfl_sync(0xffffffffu, drawn, 0);
+        draw();
+        return it;
+    };
+    draw();
+    auto cell_of = [&](int it) { return it < nitems ? items[it + 1] : make_int4(-1, 0, 0, 0); };
+    struct Head {
+        int cx, qb, nq, beg, len;  // beg, len: row r of the candidates in lane r < 9
+        float4 me;                 // lane q < nq: query qb + q
+        double z;
+        uint8_t type;
+    };
+    auto head_of = [&](int4 item) {
+        Head h{item.x, item.w, 0, 0, 0, {}, 0.0, LSMPS_WALL};
+        if (item.x < 0) return h;
+        h.nq = min(32, g.cell_start[(item.z * g.ny + item.y) * g.nx + item.x + 1] - item.w);
+        if (lane < 9) {
+            int end = 0;
+            if (row_range(g, item.x, item.y, item.z, lane % 3 - 1, lane / 3 - 1, h.beg, end)) h.len = end - h.beg;
         }
-    }
-    __syncthreads();
-    const int total = rbase[9];
-    if (total > SEG_MAXC) {
-        // crowded neighborhood: the global-memory form, one query per warp
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        for (int k = q0 + warp; k < q1; k += SEG_THREADS / 32)
-            scan_query_global(G.g, sx, sy, sz, scell, stype, k, re2, maxn, l0, classify, slots, cnt, trunc_total, cls,
-                              lane);
-        return;
-    }
-    const double ox = (G.g0.x + cx0) * G.re, oy = (G.g0.y + cy) * G.re, oz = (G.g0.z + cz0) * G.re;
-    float* fxy = reinterpret_cast<float*>(cxy);
-    float* fz = reinterpret_cast<float*>(cz);
-    for (int r = 0; r < 9; ++r) {  // row by row: consecutive threads load consecutive particles
-        const int n_r = rbase[r + 1] - rbase[r], f = rfirst[r], b = rbase[r];
-        for (int i = threadIdx.x; i < n_r; i += blockDim.x) {
-            const int si = b + i, p = si >> 1, h = si & 1;
-            fxy[4 * p + h] = (float)(sx[f + i] - ox);
-            fxy[4 * p + 2 + h] = (float)(sy[f + i] - oy);
-            fz[2 * p + h] = (float)(sz[f + i] - oz);
+        const int k = min(item.w + lane, n - 1);  // (lanes past nq load another particle's)
+        h.me = rel[k];
+        if (classify) h.type = stype[k], h.z = sz[k];
+        return h;
+    };
+    Head next = head_of(cell_of(first));
+    int4 item1 = cell_of(after());
+    while (next.nq > 0) {
+        const Head H = next;
+        next = head_of(item1);
+        item1 = cell_of(after());
+        const int cx = H.cx, qb = H.qb, nq = H.nq;
+        int pre = H.len;
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, pre, o);
+            if (lane >= o) pre += v;
         }
-    }
-    __syncthreads();
-    for (int k = q0 + threadIdx.x; k < q1; k += blockDim.x) {
-        const int ck = scell[k] - rowlin;                   // the query's cell along x
-        const int kst = rbase[4] + (k - rfirst[4]);         // the query staged in the centre row
-        const float qxs = fxy[4 * (kst >> 1) + (kst & 1)], qys = fxy[4 * (kst >> 1) + 2 + (kst & 1)];
-        const float qzs = fz[2 * (kst >> 1) + (kst & 1)];
-        const float2 nqx = make_float2(-qxs, -qxs), nqy = make_float2(-qys, -qys), nqz = make_float2(-qzs, -qzs);
-        const float qx = qxs - (ck - cx0) * re_f;          // position inside its own cell (x)
-        int* out = slots + (size_t)k * maxn;
+        const int total = __shfl_sync(0xffffffffu, pre, 8);
+        const int shift = H.beg - (pre - H.len);  // candidate index to particle
+        int start[9];                             // where the rows start among the candidates
+#pragma unroll
+        for (int r = 1; r < 9; ++r) start[r] = __shfl_sync(0xffffffffu, pre, r - 1);
+        // the rule reads the sectors of fluid particles above the wall layer only
+        const unsigned need = __ballot_sync(0xffffffffu, H.type != LSMPS_WALL && !(H.z < xmul(1.5, l0)));
         int written = 0;
         unsigned sec = 0;
-        for (int r = 0; r < 9; ++r) {
-            const int dy = r % 3 - 1, dz = r / 3 - 1;
-            const float gy = dy < 0 ? qys : (dy > 0 ? re_f - qys : 0.f);
-            const float gz = dz < 0 ? qzs : (dz > 0 ? re_f - qzs : 0.f);
-            const float gyz = gy * gy + gz * gz;
-            if (gyz > cull) continue;
-            // cells ck-1 .. ck+1 of this row, each kept when its box is within re
-            int clo = max(ck - 1, lo), chi = min(ck + 1, hi);
-            if (clo < ck && gyz + qx * qx > cull) clo = ck;
-            if (chi > ck && gyz + (re_f - qx) * (re_f - qx) > cull) chi = ck;
-            const int gb = rcs[r][clo - lo], ge = rcs[r][chi + 1 - lo];
-            const int sb = rbase[r] + (gb - rfirst[r]);
-            const int se = sb + (ge - gb);
-            const int mshift = rfirst[r] - rbase[r];  // global index = staged index + mshift
-            const int pend = (se + 1) >> 1;
-            for (int pb = sb >> 1; pb < pend; pb += 16) {
-                const int c0 = pb << 1;  // first staged candidate of this chunk of 32
-                const int np = min(16, pend - pb);
-                unsigned hit = 0;
+        for (int c0 = 0; c0 < total; c0 += 32 * SCAN_CH) {
+            float x[SCAN_CH], y[SCAN_CH], z[SCAN_CH];
+            int m[SCAN_CH];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    if (j < np) {
-                        const float4 a = cxy[pb + j];
-                        const float2 dxv = __fadd2_rn(make_float2(a.x, a.y), nqx);
-                        const float2 dyv = __fadd2_rn(make_float2(a.z, a.w), nqy);
-                        const float2 dzv = __fadd2_rn(cz[pb + j], nqz);
-                        float2 d2 = __fmul2_rn(dxv, dxv);
-                        d2 = __ffma2_rn(dyv, dyv, d2);
-                        d2 = __ffma2_rn(dzv, dzv, d2);
-                        if (d2.x <= hi_th) hit |= 1u << (2 * j);
-                        if (d2.y <= hi_th) hit |= 2u << (2 * j);
+            for (int c = 0; c < SCAN_CH; ++c) {
+                const int b = c0 + 32 * c, j = b + lane;
+                x[c] = y[c] = z[c] = 1e18f;  // no candidate: far away
+                m[c] = -1;
+                if (b < total) {
+                    int r = 0;
+#pragma unroll
+                    for (int t = 1; t < 9; ++t) r += j >= start[t] ? 1 : 0;
+                    const int mm = j + __shfl_sync(0xffffffffu, shift, r);
+                    if (j < total) {
+                        const float4 p = rel[mm];
+                        m[c] = mm;
+                        x[c] = p.x + (float)(__float_as_int(p.w) - cx) * re_f;
+                        y[c] = p.y + (float)(r % 3 - 1) * re_f;
+                        z[c] = p.z + (float)(r / 3 - 1) * re_f;
                     }
-                }
-                // keep the window [sb, se) and drop the query itself
-                const int wlo = sb - c0, whi = se - c0;
-                if (whi < 32) hit &= (1u << whi) - 1u;
-                if (wlo > 0) hit &= ~((1u << wlo) - 1u);
-                if (r == 4 && kst >= c0 && kst < c0 + 32) hit &= ~(1u << (kst - c0));
-                while (hit) {
-                    const int i = __ffs(hit) - 1;
-                    hit &= hit - 1;
-                    const int si = c0 + i, p = si >> 1, h = si & 1;
-                    const float dx = fxy[4 * p + h] - qxs, dyf = fxy[4 * p + 2 + h] - qys, dzf = fz[2 * p + h] - qzs;
-                    const float d2 = dx * dx + dyf * dyf + dzf * dzf;
-                    const int m = si + mshift;
-                    if (d2 >= lo_th && !(xnorm2(xsub(sx[m], sx[k]), xsub(sy[m], sy[k]), xsub(sz[m], sz[k])) < re2))
-                        continue;
-                    if (written < maxn) {
-                        out[written] = m;
-                        if (classify) {
-                            unsigned bb;
-                            if (!sector_bits_f32(dx, dyf, dzf, margin, bb))
-                                bb = sector_bits(xsub(sx[m], sx[k]), xsub(sy[m], sy[k]), xsub(sz[m], sz[k]));
-                            sec |= bb;
-                        }
-                    }
-                    ++written;
                 }
             }
+            // two queries at a time, so that one's chain of ballot, packing and sector bits fills the
+            // other's waits (an odd last query goes twice, the second time without results)
+            for (int q = 0; q < nq; q += 2) {
+                float qx[2], qy[2], qz[2], near = re2f;
+                unsigned bal[2][SCAN_CH];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int from = min(q + h, nq - 1);
+                    qx[h] = __shfl_sync(0xffffffffu, H.me.x, from);
+                    qy[h] = __shfl_sync(0xffffffffu, H.me.y, from);
+                    qz[h] = __shfl_sync(0xffffffffu, H.me.z, from);
+                }
+#pragma unroll
+                for (int c = 0; c < SCAN_CH; c += 2) {
+                    bal[0][c] = bal[0][c + 1] = bal[1][c] = bal[1][c + 1] = 0;
+                    if (c0 + 32 * c < total) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const float2 dx = __fadd2_rn(make_float2(x[c], x[c + 1]), make_float2(-qx[h], -qx[h]));
+                            const float2 dy = __fadd2_rn(make_float2(y[c], y[c + 1]), make_float2(-qy[h], -qy[h]));
+                            const float2 dz = __fadd2_rn(make_float2(z[c], z[c + 1]), make_float2(-qz[h], -qz[h]));
+                            float2 d2 = __fmul2_rn(dx, dx);
+                            d2 = __ffma2_rn(dy, dy, d2);
+                            d2 = __ffma2_rn(dz, dz, d2);
+                            const float2 o = __fadd2_rn(d2, make_float2(-re2f, -re2f));
+                            near = fminf(near, fminf(fabsf(o.x), fabsf(o.y)));
+                            bal[h][c] = __ballot_sync(0xffffffffu, d2.x <= hi_th && m[c] != qb + q + h);
+                            bal[h][c + 1] = __ballot_sync(0xffffffffu, d2.y <= hi_th && m[c + 1] != qb + q + h);
+                        }
+                    }
+                }
+                if (__any_sync(0xffffffffu, near <= band)) {
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) {
+                        const int kq = qb + min(q + h, nq - 1);
+#pragma unroll
+                        for (int c = 0; c < SCAN_CH; ++c) {
+                            const unsigned old = h ? bal[1][c] : bal[0][c];
+                            bool ok = (old >> lane) & 1u;
+                            if (ok) {
+                                const float dx = x[c] - (h ? qx[1] : qx[0]), dy = y[c] - (h ? qy[1] : qy[0]),
+                                            dz = z[c] - (h ? qz[1] : qz[0]);
+                                if (dx * dx + dy * dy + dz * dz >= lo_th)
+                                    ok = xnorm2(xsub(sx[m[c]], sx[kq]), xsub(sy[m[c]], sy[kq]),
+                                                xsub(sz[m[c]], sz[kq])) < re2;
+                            }
+                            const unsigned now = __ballot_sync(0xffffffffu, ok);
+                            if (h) bal[1][c] = now;
+                            else bal[0][c] = now;
+                        }
+                    }
+                }
+                int w[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    w[h] = 0;
+#pragma unroll
+                    for (int c = 0; c < SCAN_CH; ++c) {
+                        if ((bal[h][c] >> lane) & 1u)
+                            hits[h * 32 * SCAN_CH + w[h] + __popc(bal[h][c] & lt)] =
+                                make_float4(x[c], y[c], z[c], __int_as_float(m[c]));
+                        w[h] += __popc(bal[h][c]);
+                    }
+                }
+                __syncwarp();
+                const bool two = q + 1 < nq;
+                unsigned sb[2] = {0, 0};
+                int w0[2];
+                w0[0] = __shfl_sync(0xffffffffu, written, q);
+                w0[1] = __shfl_sync(0xffffffffu, written, min(q + 1, 31));
+                const int most = max(w[0], two ? w[1] : 0);
+                for (int e = lane; e < most; e += 32) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (e < w[h] && e < maxn - w0[h] && (h == 0 || two)) {
+                            const int kq = qb + q + h;
+                            const float4 f = hits[h * 32 * SCAN_CH + e];
+                            const int mh = __float_as_int(f.w);
+                            slots[(size_t)kq * maxn + w0[h] + e] = mh;
+                            unsigned bb;
+                            if (!sector_bits_f32(f.x - qx[h], f.y - qy[h], f.z - qz[h], margin, bb) &&
+                                ((need >> (q + h)) & 1u))
+                                bb = sector_bits(xsub(sx[mh], sx[kq]), xsub(sy[mh], sy[kq]), xsub(sz[mh], sz[kq]));
+                            sb[h] |= bb;
+                        }
+                    }
+                }
+                const unsigned s0 = __reduce_or_sync(0xffffffffu, sb[0]), s1 = __reduce_or_sync(0xffffffffu, sb[1]);
+                if (lane == q) {
+                    written += w[0];
+                    sec |= s0;
+                }
+                if (lane == q + 1 && two) {
+                    written += w[1];
+                    sec |= s1;
+                }
+                __syncwarp();
+            }
         }
-        cnt[k] = min(written, maxn);
-        if (written > maxn) atomicAdd(trunc_total, (unsigned long long)(written - maxn));
-        if (classify) cls[k] = classify_rule(stype[k], min(written, maxn), sec, sz[k], l0);
+        if (lane < nq) {
+            const int k = qb + lane;
+            cnt[k] = min(written, maxn);
+            if (written > maxn) atomicAdd(trunc_total, (unsigned long long)(written - maxn));
+            if (classify) cls[k] = classify_rule(H.type, min(written, maxn), sec, H.z, l0);
+        }
     }
 }
 
@@ -748,55 +809,64 @@ __global__ void __launch_bounds__(256) k_slots_compact(int n, int maxn, const in
     for (int p = sub; p < c; p += 8) col[b + p] = __ldcs(src + p);
 }
 
-// Refresh of skin lists in one pass (warp per particle): the candidates j != i of the candidate
-// CSR (radius re + skin, ascending sorted index) that pass the build's exact FP64 test
+// Refresh of skin lists in one pass (eight lanes per particle): the candidates j != i of the
+// candidate CSR (radius re + skin, ascending sorted index) that pass the build's exact FP64 test
 // |r_j - r_i|^2 < re^2, in candidate order, go to the particle's slot row (the first maxn),
 // with the sector bits of the kept ones for the classification; counting continues past maxn.
+// The sector bits come from the FP32 rounding of the FP64 differences when every comparison
+// they need is separated by more than `margin` (1e-6 re, the differences being below re and
+// rounded to 6e-8 of themselves), else from the FP64 ones.
+// Bound by instruction issue (70 % of the slots): with a warp per particle and the sector bits in
+// FP64 it took 1,665 us for 3M particles (1,260 now).
 __global__ void __launch_bounds__(256) k_filter_slots(int n, const int* __restrict__ crow,
                                                       const int* __restrict__ ccol, const double* __restrict__ sx,
                                                       const double* __restrict__ sy, const double* __restrict__ sz,
-                                                      const uint8_t* __restrict__ stype, double re2, int maxn,
-                                                      double l0, int classify, int* __restrict__ slots,
+                                                      const uint8_t* __restrict__ stype, double re2, float margin,
+                                                      int maxn, double l0, int classify, int* __restrict__ slots,
                                                       int* __restrict__ cnt, unsigned long long* trunc,
                                                       uint8_t* __restrict__ cls) {
-    const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    const int nw = (int)((gridDim.x * (size_t)blockDim.x) >> 5);
-    for (int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5); i < n; i += nw) {
+    const int lane = threadIdx.x & 31, sub = lane & 7;
+    const long long step = (gridDim.x * (long long)blockDim.x) >> 3;
+    // (the four particles of a warp go round together)
+    for (long long i0 = (blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31)) >> 3; i0 < n; i0 += step) {
+        const bool live = i0 + (lane >> 3) < n;
+        const int i = live ? (int)(i0 + (lane >> 3)) : n - 1;
         const double xi = sx[i], yi = sy[i], zi = sz[i];
-        const int c0 = crow[i], c1 = crow[i + 1];
+        const int c0 = crow[i], c1 = live ? crow[i + 1] : c0;
         int* out = slots + (size_t)i * maxn;
         int kept = 0;
         unsigned sec = 0;
-        for (int b = c0; b < c1; b += 32) {
-            const int e = b + lane;
-            bool ok = false;
-            int j = 0;
+        const int steps = __reduce_max_sync(0xffffffffu, (c1 - c0 + 7) >> 3);
+        int jnext = c0 + sub < c1 ? ccol[c0 + sub] : 0;  // loaded one step ahead of its position
+        for (int t = 0, e = c0 + sub; t < steps; ++t, e += 8) {
+            const int j = jnext;
+            jnext = e + 8 < c1 ? ccol[e + 8] : 0;
+            bool ok = e < c1 && j != i;
             double dx = 0, dy = 0, dz = 0;
-            if (e < c1) {
-                j = ccol[e];
+            if (ok) {
                 dx = xsub(sx[j], xi);
                 dy = xsub(sy[j], yi);
                 dz = xsub(sz[j], zi);
-                ok = j != i && xnorm2(dx, dy, dz) < re2;
+                ok = xnorm2(dx, dy, dz) < re2;
             }
-            const unsigned m = __ballot_sync(0xffffffffu, ok);
-            if (ok) {
-                const int p = kept + __popc(m & lt);
-                if (p < maxn) {
-                    out[p] = j;
-                    if (classify) sec |= sector_bits(dx, dy, dz);
+            const unsigned m = (__ballot_sync(0xffffffffu, ok) >> (lane & 24)) & 0xffu;
+            const int p = kept + __popc(m & ((1u << sub) - 1u));
+            if (ok && p < maxn) {
+                out[p] = j;
+                if (classify) {
+                    unsigned bb;
+                    if (!sector_bits_f32((float)dx, (float)dy, (float)dz, margin, bb)) bb = sector_bits(dx, dy, dz);
+                    sec |= bb;
                 }
             }
             kept += __popc(m);
         }
-        if (lane == 0) {
+        if (classify)
+            for (int o = 4; o; o >>= 1) sec |= __shfl_xor_sync(0xffffffffu, sec, o);
+        if (live && sub == 0) {
             cnt[i] = min(kept, maxn);
             if (kept > maxn) atomicAdd(trunc, (unsigned long long)(kept - maxn));
-        }
-        if (classify) {
-            sec = __reduce_or_sync(0xffffffffu, sec);
-            if (lane == 0) cls[i] = classify_rule(stype[i], min(kept, maxn), sec, zi, l0);
+            if (classify) cls[i] = classify_rule(stype[i], min(kept, maxn), sec, zi, l0);
         }
     }
 }
@@ -922,6 +992,51 @@ void nb_stats(lsmps_ctx* ctx, lsmps_neighbor_stats* out, const char* where) {
     fill_stats(ctx, h, out);
 }
 
+static GridView grid_view(lsmps_ctx* ctx) {
+    return {ctx->cell_start.get<int>(), ctx->gdim[0], ctx->gdim[1], ctx->gdim[2]};
+}
+
+// The two passes' non-empty segments, listed in ctx->seg_list
+static SegGrid list_segments(lsmps_ctx* ctx) {
+    cudaStream_t s = ctx->stream;
+    const SegGrid sg{grid_view(ctx), make_int3(ctx->gmin[0], ctx->gmin[1], ctx->gmin[2]), ctx->re,
+                     (ctx->gdim[0] + SEG - 1) / SEG};
+    const long long nseg = (long long)sg.nsegx * ctx->gdim[1] * ctx->gdim[2];
+    int* list = ctx->seg_list.ensure<int>(nseg + 1);
+    int* count = ctx->scratch.get<int>() + 40;
+    LSMPS_CUDA(cudaMemsetAsync(count, 0, sizeof(int), s));
+    k_list_segments<<<(unsigned)((nseg + 255) / 256), 256, 0, s>>>(sg, nseg, list, count);
+    LSMPS_CHECK_LAUNCH();
+    read_back(ctx, {{count, &ctx->nsegs, sizeof(int)}}, nullptr);
+    return sg;
+}
+
+// The single pass's items and relative positions
+static void scan_prep(lsmps_ctx* ctx) {
+    cudaStream_t s = ctx->stream;
+    const size_t n = ctx->n;
+    const size_t most = std::min((size_t)ctx->ncells, n) + n / 32 + 1;  // non-empty cells, and their further blocks
+    int4* items = ctx->scan_items.ensure<int4>(most + 1);
+    float4* rel = ctx->scan_rel.ensure<float4>(n);
+    LSMPS_CUDA(cudaMemsetAsync(items, 0, sizeof(int4), s));
+    k_scan_prep<<<blocks_for(std::max(n, (size_t)ctx->ncells), 256), 256, 0, s>>>(
+        grid_view(ctx), make_int3(ctx->gmin[0], ctx->gmin[1], ctx->gmin[2]), ctx->re, ctx->ncells, (int)n,
+        ctx->scell.get<int>(), ctx->sx.get<double>(), ctx->sy.get<double>(), ctx->sz.get<double>(), items, rel);
+    LSMPS_CHECK_LAUNCH();
+}
+
+static void launch_cell_scan(lsmps_ctx* ctx, int maxn, double l0, int classify, int* cnt, unsigned long long* trunc,
+                             int* slots, uint8_t* cls, bool again = false) {
+    const size_t n = ctx->n, most = std::min((size_t)ctx->ncells, n) + n / 32 + 1;
+    const unsigned grid = (unsigned)std::min<size_t>((most + SCAN_WARPS - 1) / SCAN_WARPS, 148 * 4);
+    if (again) LSMPS_CUDA(cudaMemsetAsync(&ctx->scan_items.get<int4>()->y, 0, sizeof(int), ctx->stream));
+    k_cell_scan<<<grid, 32 * SCAN_WARPS, 0, ctx->stream>>>(
+        grid_view(ctx), (int)n, ctx->scan_items.get<int4>(), ctx->scan_rel.get<float4>(), ctx->sx.get<double>(),
+        ctx->sy.get<double>(), ctx->sz.get<double>(), ctx->stype.get<uint8_t>(), (float)ctx->re, ctx->re2, maxn, l0,
+        classify, cnt, trunc, slots, cls);
+    LSMPS_CHECK_LAUNCH();
+}
+
 void nb_build(lsmps_ctx* ctx, double re, int maxn, double l0, int flags, lsmps_neighbor_stats* out) {
     LSMPS_REQUIRE(re > 0 && std::isfinite(re), LSMPS_ERR_ARG, "re must be positive and finite");
     LSMPS_REQUIRE(maxn >= 0 && maxn <= 8192, LSMPS_ERR_ARG, "max_neighbors must be in [0, 8192]");
@@ -1005,19 +1120,6 @@ void nb_build(lsmps_ctx* ctx, double re, int maxn, double l0, int flags, lsmps_n
     int* row = ctx->nbr_row.ensure<int>(n + 1);
     unsigned long long* trunc_d = reinterpret_cast<unsigned long long*>(ctx->scratch.get<int>() + 16);
     LSMPS_CUDA(cudaMemsetAsync(trunc_d, 0, sizeof(unsigned long long), s));
-    GridView gv{cstart, gd.x, gd.y, gd.z};
-    SegGrid sg{gv, g0, re, (gd.x + SEG - 1) / SEG};
-    const long long nseg = (long long)sg.nsegx * gd.y * gd.z;
-    LSMPS_REQUIRE(nseg < (1ll << 31), LSMPS_ERR_GRID, "too many cell segments");
-    int* seg_list = ctx->seg_list.ensure<int>(nseg + 1);
-    int* seg_count = ctx->scratch.get<int>() + 40;
-    LSMPS_CUDA(cudaMemsetAsync(seg_count, 0, sizeof(int), s));
-    k_list_segments<<<(unsigned)((nseg + 255) / 256), 256, 0, s>>>(sg, nseg, seg_list, seg_count);
-    LSMPS_CHECK_LAUNCH();
-    int hsegs = 0;
-    read_back(ctx, {{seg_count, &hsegs, sizeof(int)}}, nullptr);
-    ctx->nsegs = hsegs;
-    const unsigned seg_grid = (unsigned)std::max(hsegs, 1);
     const int do_cls = (flags & LSMPS_NBR_CLASSIFY) ? 1 : 0;
     uint8_t* cls = ctx->cls.ensure<uint8_t>(n);
     // one pass into maxn slots per particle while they fit (the usual case: 0.5 GB at 1M
@@ -1025,14 +1127,15 @@ void nb_build(lsmps_ctx* ctx, double re, int maxn, double l0, int flags, lsmps_n
     const bool single = !(flags & LSMPS_NBR_TWO_PASS) && (double)n * (double)maxn * 4.0 <= SLOT_BUDGET_BYTES;
     ctx->nbr_single = single;
     int* slots = single ? ctx->nbr_slots.ensure<int>((size_t)n * maxn + 1) : nullptr;
-    if (n && hsegs) {
-        if (single)
-            k_seg_scan<<<seg_grid, SEG_THREADS, 0, s>>>(sg, seg_list, sx, sy, sz, scell, stype, ctx->re2, maxn, l0,
-                                                       do_cls, cnt, trunc_d, slots, cls);
-        else
-            k_seg_pass<false><<<seg_grid, SEG_THREADS, 0, s>>>(sg, seg_list, sx, sy, sz, scell, stype,
-                                                                 ctx->re2, maxn, l0, 0, cnt, trunc_d, nullptr, nullptr,
-                                                                 nullptr);
+    SegGrid sg{};
+    if (n && single) {
+        scan_prep(ctx);
+        launch_cell_scan(ctx, maxn, l0, do_cls, cnt, trunc_d, slots, cls);
+    } else if (n) {
+        sg = list_segments(ctx);
+        k_seg_pass<false><<<(unsigned)ctx->nsegs, SEG_THREADS, 0, s>>>(sg, ctx->seg_list.get<int>(), sx, sy, sz, scell,
+                                                                       stype, ctx->re2, maxn, l0, 0, cnt, trunc_d,
+                                                                       nullptr, nullptr, nullptr);
         LSMPS_CHECK_LAUNCH();
     }
     scan_exclusive<int>(cnt, row, (long long)n, s, ctx->scan_tmp, dflag);
@@ -1044,13 +1147,13 @@ void nb_build(lsmps_ctx* ctx, double re, int maxn, double l0, int flags, lsmps_n
     ctx->truncated = htr;
     ctx->max_cell_occupancy = hocc;
     int* col = ctx->nbr_col.ensure<int>((size_t)hpairs + 1);
-    if (n && hsegs) {
+    if (n) {
         if (single)
             k_slots_compact<<<(unsigned)((8ull * n + 255) / 256), 256, 0, s>>>((int)n, maxn, slots, row, col);
         else
-            k_seg_pass<true><<<seg_grid, SEG_THREADS, 0, s>>>(sg, seg_list, sx, sy, sz, scell, stype,
-                                                                ctx->re2, maxn, l0, do_cls, nullptr, nullptr, row, col,
-                                                                cls);
+            k_seg_pass<true><<<(unsigned)ctx->nsegs, SEG_THREADS, 0, s>>>(sg, ctx->seg_list.get<int>(), sx, sy, sz,
+                                                                          scell, stype, ctx->re2, maxn, l0, do_cls,
+                                                                          nullptr, nullptr, row, col, cls);
         LSMPS_CHECK_LAUNCH();
     }
     ctx->have_neighbors = true;
@@ -1073,11 +1176,11 @@ bool nb_filter_single(lsmps_ctx* ctx, int classify) {
     auto* trunc_d = reinterpret_cast<unsigned long long*>(ctx->scratch.get<int>() + 16);
     LSMPS_CUDA(cudaMemsetAsync(trunc_d, 0, sizeof(unsigned long long), s));
     if (n) {
-        const unsigned grid = std::max(1u, std::min<unsigned>(blocks_for(n * 32, 256), 148 * 16));
+        const unsigned grid = std::max(1u, std::min<unsigned>(blocks_for(n * 8, 256), 148 * 64));
         k_filter_slots<<<grid, 256, 0, s>>>((int)n, ctx->cand_row.get<int>(), ctx->cand_col.get<int>(),
                                             ctx->sx.get<double>(), ctx->sy.get<double>(), ctx->sz.get<double>(),
-                                            ctx->stype.get<uint8_t>(), ctx->re2, maxn, ctx->l0, classify, slots, cnt,
-                                            trunc_d, cls);
+                                            ctx->stype.get<uint8_t>(), ctx->re2, (float)(1e-6 * ctx->re), maxn, ctx->l0,
+                                            classify, slots, cnt, trunc_d, cls);
         LSMPS_CHECK_LAUNCH();
     }
     scan_exclusive<int>(cnt, row, (long long)n, s, ctx->scan_tmp, dflag);
@@ -1098,11 +1201,13 @@ void nb_kernel_bench(lsmps_ctx* ctx, int kernel, int reps, double* ms, double* b
     LSMPS_REQUIRE(ctx->have_neighbors, LSMPS_ERR_STATE, "kernel bench needs neighbor lists");
     cudaStream_t s = ctx->stream;
     int n = (int)ctx->n;
-    GridView gv{ctx->cell_start.get<int>(), ctx->gdim[0], ctx->gdim[1], ctx->gdim[2]};
-    SegGrid sg{gv, make_int3(ctx->gmin[0], ctx->gmin[1], ctx->gmin[2]), ctx->re, (ctx->gdim[0] + SEG - 1) / SEG};
     auto* trunc_d = reinterpret_cast<unsigned long long*>(ctx->scratch.get<int>() + 16);
+    if (n == 0) { *ms = 0; *bytes = 0; return; }
+    SegGrid sg{};
+    if (kernel == LSMPS_KB_NBR_SCAN) scan_prep(ctx);
+    else if (kernel != LSMPS_KB_NBR_COMPACT) sg = list_segments(ctx);
     const int* seg_list = ctx->seg_list.get<int>();
-    const unsigned seg_grid = (unsigned)std::max(ctx->nsegs, 1);
+    const unsigned seg_grid = (unsigned)ctx->nsegs;
     int* slots = nullptr;
     if (kernel == LSMPS_KB_NBR_SCAN || kernel == LSMPS_KB_NBR_COMPACT) {
         LSMPS_REQUIRE((double)n * (double)ctx->maxn * 4.0 <= SLOT_BUDGET_BYTES, LSMPS_ERR_STATE,
@@ -1113,10 +1218,8 @@ void nb_kernel_bench(lsmps_ctx* ctx, int kernel, int reps, double* ms, double* b
     }
     auto launch = [&] {
         if (kernel == LSMPS_KB_NBR_SCAN)
-            k_seg_scan<<<seg_grid, SEG_THREADS, 0, s>>>(
-                sg, seg_list, ctx->sx.get<double>(), ctx->sy.get<double>(), ctx->sz.get<double>(), ctx->scell.get<int>(),
-                ctx->stype.get<uint8_t>(), ctx->re2, ctx->maxn, ctx->l0, ctx->have_classes ? 1 : 0,
-                ctx->nbr_cnt.get<int>(), trunc_d, slots, ctx->cls.get<uint8_t>());
+            launch_cell_scan(ctx, ctx->maxn, ctx->l0, ctx->have_classes ? 1 : 0, ctx->nbr_cnt.get<int>(), trunc_d, slots,
+                             ctx->cls.get<uint8_t>(), true);
         else if (kernel == LSMPS_KB_NBR_COMPACT)
             k_slots_compact<<<(unsigned)((8ull * n + 255) / 256), 256, 0, s>>>(n, ctx->maxn, slots,
                                                                                ctx->nbr_row.get<int>(),
@@ -1133,7 +1236,6 @@ void nb_kernel_bench(lsmps_ctx* ctx, int kernel, int reps, double* ms, double* b
                 ctx->nbr_row.get<int>(), ctx->nbr_col.get<int>(), ctx->cls.get<uint8_t>());
         LSMPS_CHECK_LAUNCH();
     };
-    if (n == 0 || ctx->nsegs == 0) { *ms = 0; *bytes = 0; return; }
     launch();  // warm
     ev_record(ctx, 14);
     for (int r = 0; r < reps; ++r) launch();
