@@ -112,14 +112,15 @@ __global__ void k_ppe_exact(size_t n, int variant, const double* __restrict__ sx
 }
 
 // One pass over the rows, PPE_G lanes per row: the lanes of a row's group take its neighbors
-// PPE_G at a time and compute their coefficients; every lane then replays the group's
-// coefficients in neighbor order, so the diagonal and b = A p* are the sequential sums of
-// the reference's order (exact FP64 operations), identical in all lanes. Kept off-diagonal
+// PPE_G at a time and compute their coefficients; one lane then adds the group's coefficients
+// in neighbor order and another its terms of b, so the diagonal and b = A p* are the sequential
+// sums of the reference's order (exact FP64 operations). Kept off-diagonal
 // entries go, in order, to the row's slot range at nbr_row[k] + k (room for every neighbor
 // plus the diagonal); k_ppe_pack moves them into the CSR once the row lengths are scanned.
 // Writes cnt[u] (entries with the diagonal), p*[u], b[u], D^-1[u].
-// stats (u64): [0] neumann, [1] failed rows. Capped at 64 registers (8 blocks of 128 threads
-// per SM; 72 uncapped): 0.80 against 0.82 ms for the assembly at 1M particles.
+// stats (u64): [0] neumann, [1] failed rows. Bound by instruction issue (67 %): with the terms
+// passed by shuffles and added in every lane 470 us at 911k unknowns (417 now) and 897 at the
+// 3M rain series (803). Capped at 64 registers (8 blocks of 128 threads per SM).
 constexpr int PPE_G = 8;
 __global__ void __launch_bounds__(128, 8) k_ppe_rows(PpeParams P, long long U, const int* __restrict__ sorted_of_u,
                                                   const int* __restrict__ ref_of_u, const int* __restrict__ uidx,
@@ -131,8 +132,10 @@ __global__ void __launch_bounds__(128, 8) k_ppe_rows(PpeParams P, long long U, c
                                                   int* __restrict__ scol, double* __restrict__ sval,
                                                   const double* __restrict__ xep, double* __restrict__ xexact,
                                                   double* __restrict__ b,
-                                                  double* __restrict__ dinv, unsigned long long* stats) {
-    const int lane = threadIdx.x & 31, sub = lane & (PPE_G - 1), gbase = lane & ~(PPE_G - 1);
+                                                  double* __restrict__ dinv, long long* __restrict__ src,
+                                                  unsigned long long* stats) {
+    __shared__ double terms[4][32][2];
+    const int lane = threadIdx.x & 31, sub = lane & (PPE_G - 1), gbase = lane & ~(PPE_G - 1), warp = threadIdx.x >> 5;
     const long long u = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / PPE_G;
     const bool live = u < U;
     int k = 0, e0 = 0, e1 = 0;
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(128, 8) k_ppe_rows(PpeParams P, long long U, c
     const long long sbase = live ? (long long)row[k] + k : 0;  // the row's slot range
     // the warp walks the longest of its groups' rows; shorter rows idle (flags stay 0)
     const int chunks = __reduce_max_sync(0xffffffffu, (e1 - e0 + PPE_G - 1) / PPE_G);
-    double diag = 0.0, bsum = 0.0;
+    double sum = 0.0;
     int written = 0;
     // the neighbor index of the next chunk is loaded one chunk ahead, so each chunk waits for
     // one round trip (its gathers) instead of two
@@ -189,16 +192,16 @@ __global__ void __launch_bounds__(128, 8) k_ppe_rows(PpeParams P, long long U, c
             sval[p] = -a;
         }
         written += __popc(kb);
-        // the group's coefficients in neighbor order: diagonal and b as sequential sums
+        // the group's terms in neighbor order: the diagonal in its first lane and b in its second,
+        // as sequential sums (a pair without a term adds +0, which changes no sum of these)
+        terms[warp][gbase + sub][0] = contrib ? a : 0.0;
+        terms[warp][gbase + sub][1] = keep ? xmul(-a, xem) : 0.0;
+        __syncwarp();
 #pragma unroll
-        for (int j = 0; j < PPE_G; ++j) {
-            const double aj = __shfl_sync(0xffffffffu, a, gbase + j);
-            const double xj = __shfl_sync(0xffffffffu, xem, gbase + j);
-            const int fj = __shfl_sync(0xffffffffu, (contrib ? 1 : 0) | (keep ? 2 : 0), gbase + j);
-            if (fj & 1) diag = xadd(diag, aj);
-            if (fj & 2) bsum = xadd(bsum, xmul(-aj, xj));
-        }
+        for (int j = 0; j < PPE_G; ++j) sum = xadd(sum, terms[warp][gbase + j][sub & 1]);
+        __syncwarp();
     }
+    double diag = __shfl_sync(0xffffffffu, sum, gbase), bsum = __shfl_sync(0xffffffffu, sum, gbase + 1);
     int neumann = 0, failed = 0;
     if (live) {
         const double xe = xep[k];
@@ -228,6 +231,7 @@ __global__ void __launch_bounds__(128, 8) k_ppe_rows(PpeParams P, long long U, c
             scol[sbase + c] = (int)u;
             sval[sbase + c] = diag;
             cnt[u] = c + 1;
+            src[u] = sbase;
             xexact[u] = xe;
             b[u] = xadd(bsum, xmul(diag, xe));
             dinv[u] = 1.0 / diag;
@@ -248,8 +252,8 @@ __global__ void __launch_bounds__(128, 8) k_ppe_rows(PpeParams P, long long U, c
 // then the block writes the range with consecutive stores. A block whose range exceeds
 // PACK_CAP entries copies its rows directly.
 constexpr int PACK_ROWS = 32, PACK_CAP = 2048, PACK_THREADS = 256;
-__global__ void __launch_bounds__(PACK_THREADS) k_ppe_pack(long long U, const int* __restrict__ sorted_of_u,
-                                                           const int* __restrict__ nrow, const int* __restrict__ arow,
+__global__ void __launch_bounds__(PACK_THREADS) k_ppe_pack(long long U, const long long* __restrict__ src,
+                                                           const int* __restrict__ arow,
                                                            const int* __restrict__ scol,
                                                            const double* __restrict__ sval, int* __restrict__ acol,
                                                            double* __restrict__ aval) {
@@ -260,10 +264,7 @@ __global__ void __launch_bounds__(PACK_THREADS) k_ppe_pack(long long U, const in
     const long long u0 = blockIdx.x * (long long)PACK_ROWS;
     const int nr = (int)min((long long)PACK_ROWS, U - u0);
     if (threadIdx.x <= nr) roff[threadIdx.x] = arow[u0 + threadIdx.x];
-    if (threadIdx.x < nr) {
-        const int k = sorted_of_u[u0 + threadIdx.x];
-        rsrc[threadIdx.x] = (long long)nrow[k] + k;
-    }
+    if (threadIdx.x < nr) rsrc[threadIdx.x] = src[u0 + threadIdx.x];
     __syncthreads();
     const int base = roff[0], total = roff[nr] - base;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -385,7 +386,8 @@ void ppe_assemble(lsmps_ctx* ctx, const lsmps_ppe_opts* o, lsmps_ppe_stats* out)
                   LSMPS_ERR_ARG, "PPE flags: LSMPS_PPE_WALL_NEUMANN is for the WLS variant");
     const int neumann = (o->flags & LSMPS_PPE_WALL_NEUMANN) ? 1 : 0;
     PpeParams P{o->variant, o->re, o->l0, o->diag_shift, 0, neumann};
-    int* cnt = ctx->vtmp.ensure<int>(U + 1);
+    auto* src = reinterpret_cast<long long*>(ctx->vtmp.ensure<char>((U + 1) * 12));  // where each row's slots start
+    int* cnt = reinterpret_cast<int*>(src + U + 1);
     int* arow = ctx->A_row.ensure<int>(U + 1);
     const int* wst = ctx->have_wls ? ctx->wls_status.get<int>() : nullptr;
     const double* wz = ctx->have_wls ? ctx->wls_z.get<double>() : nullptr;
@@ -406,7 +408,7 @@ void ppe_assemble(lsmps_ctx* ctx, const lsmps_ppe_opts* o, lsmps_ppe_stats* out)
         k_ppe_rows<<<blocks_for((size_t)U * PPE_G, 128), 128, 0, s>>>(
             P, U, sorted_of_u, ref_of_u, uidx, ctx->sx.get<double>(), ctx->sy.get<double>(), ctx->sz.get<double>(),
             ctx->cls.get<uint8_t>(), ctx->nbr_row.get<int>(), ctx->nbr_col.get<int>(), wst, wz, wws, cnt, scol, sval,
-            xep, xe, b, dinv, st);
+            xep, xe, b, dinv, src, st);
         LSMPS_CHECK_LAUNCH();
     }
     scan_exclusive<int>(cnt, arow, U, s, ctx->scan_tmp, dflag);
@@ -417,8 +419,7 @@ void ppe_assemble(lsmps_ctx* ctx, const lsmps_ppe_opts* o, lsmps_ppe_stats* out)
     int* acol = ctx->A_col.ensure<int>(nnz + 1);
     double* aval = ctx->A_val.ensure<double>(nnz + 1);
     if (U) {
-        k_ppe_pack<<<blocks_for((size_t)U, PACK_ROWS), PACK_THREADS, 0, s>>>(U, sorted_of_u, ctx->nbr_row.get<int>(),
-                                                                             arow, scol, sval, acol, aval);
+        k_ppe_pack<<<blocks_for((size_t)U, PACK_ROWS), PACK_THREADS, 0, s>>>(U, src, arow, scol, sval, acol, aval);
         LSMPS_CHECK_LAUNCH();
     }
     ev_record(ctx, 9);

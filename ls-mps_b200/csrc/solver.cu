@@ -504,72 +504,85 @@ __global__ void k_sell_len(long long n, long long nslices, const int* __restrict
     }
 }
 
-// All SELL arrays of a slice in one pass, one warp per slice of 32 rows: the slice's CSR entries
-// (one contiguous range) are staged in shared memory with coalesced loads, then each lane writes
-// its row four entries at a time with 16-byte stores: columns (the diagonal moved to its place
-// in column order, padding repeating the last column), values A (padding 0), the column steps
-// and the row's first column (any row that does not ascend or steps by more than 65535 sets
-// *bad), and the column-scaled copies A D^-1 in FP64 and FP32. Slices of more than SB_CAP
-// entries read their rows from global memory instead. Same values as a per-row fill followed
-// by the column-scaling passes (each scaled value is the same single product, rounded once).
-constexpr int SB_CAP = 1024;
-__global__ void __launch_bounds__(128) k_sell_build(long long n, long long nslices, const int* __restrict__ row,
-                                                    const int* __restrict__ acol, const double* __restrict__ aval,
-                                                    const double* __restrict__ dinv, const int* __restrict__ sptr,
-                                                    const int* __restrict__ slen, int* __restrict__ col,
-                                                    double* __restrict__ val, unsigned short* __restrict__ dcol,
-                                                    int* __restrict__ rbase, double* __restrict__ vals,
-                                                    float* __restrict__ valf, int* bad, int raw) {
-    __shared__ int scol[4][SB_CAP];
-    __shared__ double sval[4][SB_CAP];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long s = blockIdx.x * 4LL + w;
-    if (s >= nslices) return;  // whole warp
+// All SELL arrays of a slice of 32 rows in one pass, SB_WARPS warps per slice: the slice's CSR
+// entries (one contiguous range) are staged in shared memory with asynchronous copies, all in
+// flight at once, and scaled there in CSR order; then a thread writes every SB_WARPS-th group of
+// four entries of its row with 16-byte stores: columns (the diagonal moved to its place in column
+// order, padding repeating the last column), values A (padding 0), the column steps and the row's
+// first column (any row that does not ascend or steps by more than 65535 sets *bad), and the
+// column-scaled copies A D^-1 in FP64 and FP32. Slices of more than `cap` entries read their rows
+// from global memory instead. Same values as a per-row fill followed by the column-scaling passes
+// (each scaled value is the same single product, rounded once).
+// What bounds it: the copies' and the row loop's latency, so it is the number of warps per SM that
+// counts: 416 us for 911k unknowns and 102 for 181k when one warp staged a slice with one load
+// per step and slices above 1,024 entries (an interior slice has 1,056) were read in place, 286
+// and 58 with one warp and asynchronous copies, 196 and 45 with four warps (227 and 52 with two,
+// 227 and 48 with eight).
+constexpr int SB_MAX = 4000;  // entries staged at most (48 KB)
+constexpr int SB_WARPS = 4;
+template <int N>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "n"(N)
+                 : "memory");
+}
+__global__ void __launch_bounds__(32 * SB_WARPS) k_sell_build(
+    long long n, const int* __restrict__ row, const int* __restrict__ acol, const double* __restrict__ aval,
+    const double* __restrict__ dinv, const int* __restrict__ sptr, const int* __restrict__ slen, int* __restrict__ col,
+    double* __restrict__ val, unsigned short* __restrict__ dcol, int* __restrict__ rbase, double* __restrict__ vals,
+    float* __restrict__ valf, int* bad, int raw, int cap) {
+    extern __shared__ double sval[];  // cap values, then cap columns
+    int* scol = reinterpret_cast<int*>(sval + cap);
+    __shared__ int diag[32];  // where each row's diagonal goes
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long s = blockIdx.x;
     const long long u0 = s << 5, i = u0 + lane;
-    const int b0 = row[u0], b1 = row[min(u0 + 32, n)];
-    const bool staged = b1 - b0 <= SB_CAP;
-    if (staged) {
-        for (int t = lane; t < b1 - b0; t += 32) {
-            scol[w][t] = acol[b0 + t];
-            sval[w][t] = aval[b0 + t];
+    const int b0 = row[u0], b1 = row[min(u0 + 32, n)], total = b1 - b0;
+    const bool staged = total <= cap;
+    if (staged)
+        for (int t = threadIdx.x; t < total; t += 32 * SB_WARPS) {
+            copy_async<4>(scol + t, acol + b0 + t);
+            copy_async<8>(sval + t, aval + b0 + t);
         }
-    }
-    __syncwarp();
     int e0 = 0, len = 0;
     if (i < n) {
         e0 = row[i];
         len = row[i + 1] - e0;
     }
-    auto C = [&](int e) { return staged ? scol[w][e - b0] : acol[e]; };
-    auto V = [&](int e) { return staged ? sval[w][e - b0] : aval[e]; };
-    // the CSR row's last entry is its diagonal: it goes where it belongs in column order
-    int pos = 0;
-    if (len > 0)
-        while (pos < len - 1 && C(e0 + pos) < (int)i) ++pos;
-    int last = i < n ? (int)i : 0, prev = 0;
-    bool ok = true;
+    if (w == 0) diag[lane] = max(len - 1, 0);
     const int L = slen[s];
     const long long base = (long long)sptr[s] + 4 * lane;
-    for (int k4 = 0; k4 < L; k4 += 4) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const bool scaled = staged && !raw;  // the staged values are scaled in place
+    if (scaled)
+#pragma unroll 4
+        for (int t = threadIdx.x; t < total; t += 32 * SB_WARPS) sval[t] *= dinv[scol[t]];
+    auto C = [&](int e) { return staged ? scol[e - b0] : acol[e]; };
+    auto V = [&](int e) { return staged ? sval[e - b0] : aval[e]; };
+    // the CSR row's last entry is its diagonal: it goes before the first entry of a larger column
+    // (each warp looks at a part of the row)
+    const int part = (len + SB_WARPS - 2) / SB_WARPS;
+    for (int k = w * part; k < min((w + 1) * part, len - 1); ++k)
+        if (C(e0 + k) >= (int)i) {
+            atomicMin(&diag[lane], k);
+            break;
+        }
+    __syncthreads();
+    const int pos = diag[lane];
+    auto at = [&](int k) { return k < pos ? e0 + k : (k == pos ? e0 + len - 1 : e0 + k - 1); };  // the row's k-th entry
+    const int last = len > 0 ? C(at(len - 1)) : (i < n ? (int)i : 0);
+    bool ok = true;
+    for (int k4 = 4 * w; k4 < L; k4 += 4 * SB_WARPS) {
         int cc[4];
         double vv[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int k = k4 + j;
-            if (k < len) {
-                const int src = k < pos ? e0 + k : (k == pos ? e0 + len - 1 : e0 + k - 1);
-                cc[j] = C(src);
-                vv[j] = V(src);
-                last = cc[j];
-            } else {
-                cc[j] = last;
-                vv[j] = 0.0;
-            }
+            cc[j] = k < len ? C(at(k)) : last;
+            vv[j] = k < len ? V(at(k)) : 0.0;
         }
-        if (k4 == 0) {
-            prev = cc[0];
-            rbase[i] = cc[0];
-        }
+        if (k4 == 0) rbase[i] = cc[0];
+        int prev = k4 == 0 ? cc[0] : k4 - 1 < len ? C(at(k4 - 1)) : last;
         unsigned short dd[4];
         double sv[4];
 #pragma unroll
@@ -578,7 +591,7 @@ __global__ void __launch_bounds__(128) k_sell_build(long long n, long long nslic
             ok = ok && d >= 0 && d <= 65535;
             dd[j] = (unsigned short)(d >= 0 && d <= 65535 ? d : 0);
             prev = cc[j];
-            sv[j] = vv[j] * dinv[cc[j]];
+            sv[j] = scaled ? vv[j] : vv[j] * dinv[cc[j]];
         }
         const long long e = base + 128LL * (k4 >> 2);
         if (raw) {  // unscaled values and 32-bit columns: only the plain FP64 solver reads them
@@ -594,8 +607,6 @@ __global__ void __launch_bounds__(128) k_sell_build(long long n, long long nslic
     }
     if (!ok) atomicOr(bad, 1);
 }
-
-
 
 // cut[b]: the first slice of block b of SELL_CUTS, so that the blocks hold about the same number
 // of stored entries
@@ -886,6 +897,14 @@ void set_scalar_caps(Engine& E, int max_iter, int stall_window) {
     LSMPS_CUDA(cudaMemcpyAsync(E.S, &init, sizeof(init), cudaMemcpyHostToDevice, E.s));
 }
 
+// Entries of a slice that k_sell_build stages: a third more than the mean slice has, so that only
+// slices of unusually long rows are read in place and the others leave room for more blocks (half
+// as much again: 207 against 196 us at 911k unknowns).
+static int sell_stage_cap(lsmps_ctx* ctx) {
+    const long long mean = 32 * (ctx->nnz / std::max(ctx->U, 1LL) + 1);
+    return (int)std::min<long long>(SB_MAX, (mean + mean / 3 + 127) / 128 * 128);
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------------------
@@ -918,10 +937,11 @@ static void sell_structure(lsmps_ctx* ctx) {
     ctx->have_steps = false;
     if (ns) {
         int* bad = ctx->scratch.get<int>() + 46;
+        const int cap = sell_stage_cap(ctx);
         LSMPS_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
-        k_sell_build<<<(unsigned)((ns + 3) / 4), 128, 0, s>>>(U, ns, ctx->A_row.get<int>(), ctx->A_col.get<int>(),
+        k_sell_build<<<(unsigned)ns, 32 * SB_WARPS, cap * 12, s>>>(U, ctx->A_row.get<int>(), ctx->A_col.get<int>(),
                                                               ctx->A_val.get<double>(), ctx->A_dinv.get<double>(), sptr,
-                                                              slen, col, val, dcol, rbase, vals, valf, bad, 0);
+                                                              slen, col, val, dcol, rbase, vals, valf, bad, 0, cap);
         LSMPS_CHECK_LAUNCH();
         int hbad = 1;
         read_back(ctx, {{bad, &hbad, sizeof(int)}}, nullptr);
@@ -940,11 +960,12 @@ static void sell_raw(lsmps_ctx* ctx) {
     const long long U = ctx->U, ns = ctx->sell_nslices;
     if (ns) {
         int* bad = ctx->scratch.get<int>() + 46;
-        k_sell_build<<<(unsigned)((ns + 3) / 4), 128, 0, ctx->stream>>>(
-            U, ns, ctx->A_row.get<int>(), ctx->A_col.get<int>(), ctx->A_val.get<double>(), ctx->A_dinv.get<double>(),
+        const int cap = sell_stage_cap(ctx);
+        k_sell_build<<<(unsigned)ns, 32 * SB_WARPS, cap * 12, ctx->stream>>>(
+            U, ctx->A_row.get<int>(), ctx->A_col.get<int>(), ctx->A_val.get<double>(), ctx->A_dinv.get<double>(),
             ctx->S_ptr.get<int>(), ctx->S_len.get<int>(), ctx->S_col.get<int>(), ctx->S_val.get<double>(),
             ctx->S_dcol.get<unsigned short>(), ctx->S_rbase.get<int>(), ctx->S_vals.get<double>(),
-            ctx->S_valf.get<float>(), bad, 1);
+            ctx->S_valf.get<float>(), bad, 1, cap);
         LSMPS_CHECK_LAUNCH();
     }
     ctx->have_sell_raw = true;
