@@ -331,9 +331,10 @@ __global__ void k_mg_coarsen(long long ncap, const int* nd, const int* __restric
 }
 
 // ---- V-cycle ------------------------------------------------------------------------------
-// r1[I] = sum of z over the aggregate's rows
+// r1[I] = sum of z over the aggregate's rows, and the pre-smoothed iterate x1 = omega r1 / d
 __global__ void k_mg_restrict0(long long n1, const int* __restrict__ ustart, const double* __restrict__ z,
-                               float* __restrict__ r1, const BcgScalars* S, int need_s) {
+                               const float* __restrict__ dinv, float* __restrict__ r1, float* __restrict__ x1,
+                               const BcgScalars* S, int need_s) {
     pdl_begin();
     if (gated(S, need_s)) return;
     long long I = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -341,15 +342,19 @@ __global__ void k_mg_restrict0(long long n1, const int* __restrict__ ustart, con
     double a = 0;
     for (int i = ustart[I], e = ustart[I + 1]; i < e; ++i) a += z[i];
     r1[I] = (float)a;
+    x1[I] = MG_OMEGA * (float)a * dinv[I];
 }
 
-// Partial sum over the slots t = g, g + 4, ... of row I of A_l times the vector f, where
-// f(J) = omega r[J] dinv[J] (down: the pre-smoothed iterate) or x[J] + alpha ec[pn] (up).
-// Empty slots (nbr = -1) hold 0, so their index is clamped to 0 instead of branching, and all
-// of the row's loads are issued before the gathers that depend on them.
+// Partial sum over the slots t = g, g + 4, ... of row I of A_l times x (down: the pre-smoothed
+// iterate omega r / d, which whoever makes the level's residual writes too: formed at every slot
+// from r and 1 / d it took two gathers, 16.4 and 7.8 us against 15.7 and 7.2 for level 1's and the
+// next levels' kernels at 911k unknowns) or x + alpha P ec (up; adding ec to the children's
+// iterates where it is made saves a gather and the parents here, but lengthened every kernel's
+// chain: 10.1 against 9.5 us a level, the coarsest 12.9 against 9.8). Empty slots (nbr = -1) hold
+// 0, so their index is clamped to 0 instead of branching, and all of the row's loads are issued
+// before the gathers that depend on them.
 __device__ __forceinline__ float row_part_down(long long I, int g, const float* __restrict__ val,
-                                               const int* __restrict__ nbr, const float* __restrict__ r,
-                                               const float* __restrict__ dinv) {
+                                               const int* __restrict__ nbr, const float* __restrict__ x) {
     int J[7];
     float v[7];
 #pragma unroll
@@ -361,7 +366,7 @@ __device__ __forceinline__ float row_part_down(long long I, int g, const float* 
     }
     float s = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 7; ++k) s += v[k] * (MG_OMEGA * r[J[k]] * dinv[J[k]]);
+    for (int k = 0; k < 7; ++k) s += v[k] * x[J[k]];
     return s;
 }
 __device__ __forceinline__ float row_part_up(long long I, int g, const float* __restrict__ val,
@@ -383,29 +388,26 @@ __device__ __forceinline__ float row_part_up(long long I, int g, const float* __
     return s;
 }
 
-// Level l, four lanes per row (slots t = g mod 4): x_l[I] = omega r_l[I] / d_I and the
-// residual r_l[I] - (A_l x_l)[I] into res (the four partial sums added in a fixed tree).
+// Level l, four lanes per row (slots t = g mod 4): the residual r_l[I] - (A_l x_l)[I] into res
+// (the four partial sums added in a fixed tree).
 __global__ void k_mg_res(long long n, const float* __restrict__ val, const int* __restrict__ nbr,
-                         const float* __restrict__ dinv, const float* __restrict__ r, float* __restrict__ x,
-                         float* __restrict__ res, const BcgScalars* S, int need_s) {
+                         const float* __restrict__ r, const float* __restrict__ x, float* __restrict__ res,
+                         const BcgScalars* S, int need_s) {
     pdl_begin();
     if (gated(S, need_s)) return;
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const long long I = q >> 2;
     const int g = (int)(q & 3);
-    float s = I < n ? row_part_down(I, g, val, nbr, r, dinv) : 0.0f;
+    float s = I < n ? row_part_down(I, g, val, nbr, x) : 0.0f;
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if (I < n && g == 0) {
-        const float rI = r[I];
-        x[I] = MG_OMEGA * rI * dinv[I];
-        res[I] = rI - s;
-    }
+    if (I < n && g == 0) res[I] = r[I] - s;
 }
 
-// r_{l+1}[B] = sum of the children's residuals (octant order)
+// r_{l+1}[B] = sum of the children's residuals (octant order), x_{l+1} = omega r_{l+1} / d
 __global__ void k_mg_restrict(long long nc, const int* __restrict__ child, const float* __restrict__ res,
-                              float* __restrict__ rc, const BcgScalars* S, int need_s) {
+                              const float* __restrict__ dinvc, float* __restrict__ rc, float* __restrict__ xc,
+                              const BcgScalars* S, int need_s) {
     pdl_begin();
     if (gated(S, need_s)) return;
     const long long B = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -417,32 +419,33 @@ __global__ void k_mg_restrict(long long nc, const int* __restrict__ child, const
         if (I >= 0) a += res[I];
     }
     rc[B] = a;
+    xc[B] = MG_OMEGA * a * dinvc[B];
 }
 
-// One warp per coarse row B; four lanes per child I (octant o = lane / 4): x_l[I] and the
-// child's residual as in k_mg_res, then the eight residuals added in a fixed tree.
+// One warp per coarse row B; four lanes per child I (octant o = lane / 4): the child's residual
+// as in k_mg_res, then the eight residuals added in a fixed tree.
 __global__ void k_mg_down(long long nc, const int* __restrict__ child, const float* __restrict__ val,
-                          const int* __restrict__ nbr, const float* __restrict__ dinv, const float* __restrict__ r,
-                          float* __restrict__ x, float* __restrict__ rc, const BcgScalars* S, int need_s) {
+                          const int* __restrict__ nbr, const float* __restrict__ r, const float* __restrict__ x,
+                          const float* __restrict__ dinvc, float* __restrict__ rc, float* __restrict__ xc,
+                          const BcgScalars* S, int need_s) {
     pdl_begin();
     if (gated(S, need_s)) return;
     const long long B = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     if (B >= nc) return;  // whole warp
     const int lane = threadIdx.x & 31, g = lane & 3;
     const int I = child[8 * B + (lane >> 2)];
-    float s = I >= 0 ? row_part_down(I, g, val, nbr, r, dinv) : 0.0f;
+    float s = I >= 0 ? row_part_down(I, g, val, nbr, x) : 0.0f;
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     float res = 0.0f;
-    if (I >= 0) {
-        const float rI = r[I];
-        res = rI - s;
-        if (g == 0) x[I] = MG_OMEGA * rI * dinv[I];
-    }
+    if (I >= 0) res = r[I] - s;
     res += __shfl_xor_sync(0xffffffffu, res, 4);
     res += __shfl_xor_sync(0xffffffffu, res, 8);
     res += __shfl_xor_sync(0xffffffffu, res, 16);
-    if (lane == 0) rc[B] = res;
+    if (lane == 0) {
+        rc[B] = res;
+        xc[B] = MG_OMEGA * res * dinvc[B];
+    }
 }
 
 // Coarsest level (n <= MG_COARSE_MAX rows): Jacobi sweeps from 0 in one block of nb >= n
@@ -724,7 +727,8 @@ int mg_launches_per_apply(lsmps_ctx* ctx, bool restricted) {
 
 MgFine mg_fine(lsmps_ctx* ctx) {
     MgState& M = *ctx->mg;
-    return MgFine{M.L[1].n, M.ustart.get<int>(), M.agg0.get<int>(), M.L[1].r.get<float>()};
+    return MgFine{M.L[1].n, M.ustart.get<int>(), M.agg0.get<int>(), M.L[1].r.get<float>(), M.L[1].x.get<float>(),
+                  M.L[1].dinv.get<float>(), MG_OMEGA};
 }
 
 // out = D M z on the context stream (z, out: U doubles); gated by the solver scalars S
@@ -737,18 +741,18 @@ void mg_apply(lsmps_ctx* ctx, const double* z, double* out, const BcgScalars* S,
     MgLevel* L = M.L;
     if (!restricted)
         launch_pdl(k_mg_restrict0, grid_for(L[1].n, 256), 256, 0, s, L[1].n, M.ustart.get<int>(), z,
-                   L[1].r.get<float>(), S, need_s);
+                   L[1].dinv.get<float>(), L[1].r.get<float>(), L[1].x.get<float>(), S, need_s);
     for (int l = 1; l < Lc; ++l) {
+        MgLevel& C = L[l + 1];
         if (l == 1) {
             launch_pdl(k_mg_res, grid_for(4 * L[1].n, 256), 256, 0, s, L[1].n, L[1].val.get<float>(),
-                       L[1].nbr.get<int>(), L[1].dinv.get<float>(), L[1].r.get<float>(), L[1].x.get<float>(),
-                       L[1].e.get<float>(), S, need_s);
-            launch_pdl(k_mg_restrict, grid_for(L[2].n, 256), 256, 0, s, L[2].n, L[2].child.get<int>(),
-                       L[1].e.get<float>(), L[2].r.get<float>(), S, need_s);
+                       L[1].nbr.get<int>(), L[1].r.get<float>(), L[1].x.get<float>(), L[1].e.get<float>(), S, need_s);
+            launch_pdl(k_mg_restrict, grid_for(C.n, 256), 256, 0, s, C.n, C.child.get<int>(), L[1].e.get<float>(),
+                       C.dinv.get<float>(), C.r.get<float>(), C.x.get<float>(), S, need_s);
         } else {
-            launch_pdl(k_mg_down, grid_for(32 * L[l + 1].n, 256), 256, 0, s, L[l + 1].n, L[l + 1].child.get<int>(),
-                       L[l].val.get<float>(), L[l].nbr.get<int>(), L[l].dinv.get<float>(), L[l].r.get<float>(),
-                       L[l].x.get<float>(), L[l + 1].r.get<float>(), S, need_s);
+            launch_pdl(k_mg_down, grid_for(32 * C.n, 256), 256, 0, s, C.n, C.child.get<int>(), L[l].val.get<float>(),
+                       L[l].nbr.get<int>(), L[l].r.get<float>(), L[l].x.get<float>(), C.dinv.get<float>(),
+                       C.r.get<float>(), C.x.get<float>(), S, need_s);
         }
     }
     const int nbc = (int)std::max<long long>(32, (L[Lc].n + 31) / 32 * 32);

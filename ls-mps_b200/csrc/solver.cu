@@ -271,7 +271,10 @@ __global__ void __launch_bounds__(RB) k_bcg_p_agg(MgFine G, const double* __rest
             p[i] = pi;
             return pi;
         });
-        if (Ia + lane < Ib) G.r1[Ia + lane] = (float)a;
+        if (Ia + lane < Ib) {
+            G.r1[Ia + lane] = (float)a;
+            G.x1[Ia + lane] = G.omega * (float)a * G.dinv1[Ia + lane];
+        }
     }
 }
 
@@ -296,7 +299,10 @@ __global__ void __launch_bounds__(RB) k_bcg_s_agg(MgFine G, const double* __rest
             acc += si * si;
             return si;
         });
-        if (Ia + lane < Ib) G.r1[Ia + lane] = (float)a;
+        if (Ia + lane < Ib) {
+            G.r1[Ia + lane] = (float)a;
+            G.x1[Ia + lane] = G.omega * (float)a * G.dinv1[Ia + lane];
+        }
     }
     if (block_partials(acc, 0.0, P, &S->counter[1])) {
         double ss, unused;

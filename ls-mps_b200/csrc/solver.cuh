@@ -55,7 +55,9 @@ struct MgFine {
     long long n1;
     const int* ustart;
     const int* agg0;
-    float* r1;
+    float *r1, *x1;     // level 1's residual and pre-smoothed iterate omega r1 / d1
+    const float* dinv1;
+    float omega;
 };
 MgFine mg_fine(lsmps_ctx* ctx);
 
