@@ -51,9 +51,8 @@ sys.path.insert(0, os.path.join(ROOT, "oracle"))
 METRIC = "PPE solve ms & particle-steps/s at 1M, learned+mixed vs plain FP64 @ L2<=1e-8"
 UNIT = "particle-steps/s"
 L0, RE_RATIO, MAXN = 1.0, 2.1, 128
-# bench solver name -> (library solver, preconditioner, launch form). The multigrid solves
-# launch eagerly (use_graph 0): with ~27 short kernels per iteration, stream launches keep the
-# programmatic-dependent-launch overlap and measured ~5 % faster than the device-driven graph.
+# bench solver name -> (library solver, preconditioner, use_graph). These solvers' launches do not
+# depend on use_graph: one cooperative launch per solve, or stream launches with the multigrid.
 SOLVER_SPECS = {"fp64": ("fp64", "jacobi", 1), "jacobi": ("jacobi", "jacobi", 1), "mixed": ("mixed", "jacobi", 1),
                 "learned": ("learned", "jacobi", 1), "multigrid": ("mixed", "multigrid", 0),
                 "learned_multigrid": ("learned", "multigrid", 0)}

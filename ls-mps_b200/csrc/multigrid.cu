@@ -32,8 +32,8 @@
 // by the diagonal). Each level's down and up step is one grid-wide kernel (level 1's down step
 // two), the coarsest one block. Every sum has a fixed order, so a V-cycle is
 // deterministic and a fixed linear operator, as BiCGStab requires. The V-cycle kernels take
-// the solver's device scalars and return at once when the iteration has stopped (the gated
-// kernels of the device-driven loop), and start under programmatic dependent launch.
+// the solver's device scalars and return at once when the iteration has stopped (the host reads
+// the status once per chunk of iterations), and start under programmatic dependent launch.
 #include <cuda_fp16.h>
 
 #include <algorithm>

@@ -6,13 +6,13 @@
 //   2. a counting sort of particles into a dense cell grid (atomic slots, scan), then
 //      each cell's members sorted by particle index, so that every 3-cell x-row of the grid
 //      is one contiguous, index-ascending range of the sorted arrays;
-//   3. a count pass and a fill pass, one block per segment of 4 cells along x, one warp per
-//      particle: the block stages its 9 cell rows' candidates in shared memory, a warp tests
-//      a particle's 9 contiguous row ranges 32 candidates at a time (FP32 guard band, exact
-//      FP64 near the cutoff), and a ballot gives each accepted candidate its position. Scanning the 9 rows in (dz, dy) order with candidates in sorted order is
-//      exactly the reference's order (27 cells dz, dy, dx; ascending index in a cell), so
-//      the sorted column indices of a row ascend and the first max_neighbors are the ones
-//      the reference keeps. The fill pass fuses the classification over the kept list.
+//   3. a scan of every cell's 9 contiguous candidate rows by one warp (FP32 with a guard band,
+//      exact FP64 near the cutoff) into per-particle slot rows, packed into the CSR once the
+//      counts are scanned; or, where the slot rows would not fit, a count pass and a fill pass.
+//      Taking the 9 rows in (dz, dy) order with candidates in sorted order is exactly the
+//      reference's order (27 cells dz, dy, dx; ascending index in a cell), so the sorted column
+//      indices of a row ascend and the first max_neighbors are the ones the reference keeps.
+//      The scan (or the fill pass) fuses the classification over the kept list.
 // Distances use __dadd_rn/__dmul_rn: the reference evaluates (dx*dx + dy*dy) + dz*dz
 // without fused multiply-adds, and the acceptance test d^2 < re^2 must match at the ulp.
 #include <algorithm>
@@ -558,8 +558,8 @@ __global__ void __launch_bounds__(SEG_THREADS, 8) k_seg_pass(SegGrid G, const in
 // What bounds it: the latency of a query's chain (ballots, packing, sector bits) at 16 warps per
 // SM; two queries at a time hide half of it (one at a time took 518 us at 1M). It took the place
 // of a block per 12-cell segment with a thread per query, which was bound by shared memory (24
-// bytes per candidate pair and lane) and by the divergent walk over each thread's hits, with a
-// third to a half of the lanes idle: 532 us for 1M particles of a mixed set (479 now), 172 us for
+// bytes per candidate pair and lane) and by the divergent walk over each thread's hits, with 23
+// (mixed set) to 39 % (rain) of its warps' lanes idle: 532 us for 1M particles of a mixed set (479 now), 172 us for
 // 200k of a rain set (111) and 890 for 1M at radius 2.3 (513). Five blocks per SM (102
 // registers, spilled) took 499 us, three 565.
 constexpr int SCAN_CH = 10;     // chunks of 32 candidates in registers (a cell of side 2.1 has 250 candidates)

@@ -5,9 +5,10 @@
 Builds the workload of bench.py (case `mixed`, l0 = 1, re = 2.1, max_neighbors 128,
 WLS-Laplacian PPE) with the library, then launches the chosen kernel `reps` times through
 lsmps_kernel_bench and prints its mean time and achieved bandwidth. Under ncu, select the
-kernel with -k (spmv32/spmv64: k_bcg_v, nbr_count: k_seg_pass<0>, nbr_fill: k_seg_pass<1>,
-nbr_scan: k_seg_scan, nbr_compact: k_slots_compact, wls: k_wls_all, mpnn_layer: k_layer_fwd, mg_vcycle: regex k_mg_). mpnn_layer loads --weights. --autotune prints the
-launch shapes the autotuner timed and chose.
+kernel with -k (spmv32/spmv64: k_row_product, nbr_count: k_seg_pass<0>, nbr_fill: k_seg_pass<1>,
+nbr_scan: k_cell_scan, nbr_compact: k_slots_compact, wls: k_wls_all, mpnn_layer: k_layer_fwd,
+mg_vcycle: regex k_mg_). mpnn_layer loads --weights. --autotune prints the launch shapes the
+autotuner timed and chose.
 
     python ls-mps_b200/profile_kernels.py --step-trace learned --precond multigrid
 
@@ -45,8 +46,7 @@ def main():
                     help="also run one PPE solve to relative residual 1e-10")
     ap.add_argument("--precond", choices=["jacobi", "multigrid"], default="jacobi")
     ap.add_argument("--use-graph", type=int, default=1,
-                    help="launch form of --solve: 1 device-driven graph, 2 chunk graphs, 0 stream launches "
-                         "(0 for ncu, which does not profile kernels inside conditional graph nodes)")
+                    help="use_graph of --solve (it changes the launches of MIXED_F32 only)")
     ap.add_argument("--weights", default=WEIGHTS)
     ap.add_argument("--autotune", type=int, default=1, help="0 off (default shapes), 1 on")
     ap.add_argument("--step-trace", choices=["fp64", "jacobi", "mixed", "learned"], default=None,
