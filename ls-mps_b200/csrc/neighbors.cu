@@ -560,8 +560,9 @@ __global__ void __launch_bounds__(SEG_THREADS, 8) k_seg_pass(SegGrid G, const in
 // of a block per 12-cell segment with a thread per query, which was bound by shared memory (24
 // bytes per candidate pair and lane) and by the divergent walk over each thread's hits, with 23
 // (mixed set) to 39 % (rain) of its warps' lanes idle: 532 us for 1M particles of a mixed set (479 now), 172 us for
-// 200k of a rain set (111) and 890 for 1M at radius 2.3 (513). Five blocks per SM (102
-// registers, spilled) took 499 us, three 565.
+// 200k of a rain set (110) and 890 for 1M at radius 2.3 (496). Five blocks per SM (102
+// registers, spilled) took 499 us, three 565. The sector bits are left out where the rule does not
+// read them (walls, a third of a rain set: 513 -> 496 us).
 constexpr int SCAN_CH = 10;     // chunks of 32 candidates in registers (a cell of side 2.1 has 250 candidates)
 constexpr int SCAN_WARPS = 4;   // per block
 
@@ -768,11 +769,12 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS, 4) k_cell_scan(
                             const float4 f = hits[h * 32 * SCAN_CH + e];
                             const int mh = __float_as_int(f.w);
                             slots[(size_t)kq * maxn + w0[h] + e] = mh;
-                            unsigned bb;
-                            if (!sector_bits_f32(f.x - qx[h], f.y - qy[h], f.z - qz[h], margin, bb) &&
-                                ((need >> (q + h)) & 1u))
-                                bb = sector_bits(xsub(sx[mh], sx[kq]), xsub(sy[mh], sy[kq]), xsub(sz[mh], sz[kq]));
-                            sb[h] |= bb;
+                            if ((need >> (q + h)) & 1u) {
+                                unsigned bb;
+                                if (!sector_bits_f32(f.x - qx[h], f.y - qy[h], f.z - qz[h], margin, bb))
+                                    bb = sector_bits(xsub(sx[mh], sx[kq]), xsub(sy[mh], sy[kq]), xsub(sz[mh], sz[kq]));
+                                sb[h] |= bb;
+                            }
                         }
                     }
                 }
@@ -816,8 +818,9 @@ __global__ void __launch_bounds__(256) k_slots_compact(int n, int maxn, const in
 // The sector bits come from the FP32 rounding of the FP64 differences when every comparison
 // they need is separated by more than `margin` (1e-6 re, the differences being below re and
 // rounded to 6e-8 of themselves), else from the FP64 ones.
-// Bound by instruction issue (70 % of the slots): with a warp per particle and the sector bits in
-// FP64 it took 1,665 us for 3M particles (1,260 now).
+// Bound by instruction issue (70 % of the slots): with a warp per particle and every kept
+// candidate's sector bits in FP64 it took 1,665 us for 3M particles (997 now; 1,100 with the bits
+// of walls, which the rule does not read).
 __global__ void __launch_bounds__(256) k_filter_slots(int n, const int* __restrict__ crow,
                                                       const int* __restrict__ ccol, const double* __restrict__ sx,
                                                       const double* __restrict__ sy, const double* __restrict__ sz,
@@ -832,6 +835,9 @@ __global__ void __launch_bounds__(256) k_filter_slots(int n, const int* __restri
         const bool live = i0 + (lane >> 3) < n;
         const int i = live ? (int)(i0 + (lane >> 3)) : n - 1;
         const double xi = sx[i], yi = sy[i], zi = sz[i];
+        const uint8_t ti = classify ? stype[i] : LSMPS_WALL;
+        // the rule reads the sectors of fluid particles above the wall layer only
+        const bool need = ti != LSMPS_WALL && !(zi < xmul(1.5, l0));
         const int c0 = crow[i], c1 = live ? crow[i + 1] : c0;
         int* out = slots + (size_t)i * maxn;
         int kept = 0;
@@ -853,7 +859,7 @@ __global__ void __launch_bounds__(256) k_filter_slots(int n, const int* __restri
             const int p = kept + __popc(m & ((1u << sub) - 1u));
             if (ok && p < maxn) {
                 out[p] = j;
-                if (classify) {
+                if (need) {
                     unsigned bb;
                     if (!sector_bits_f32((float)dx, (float)dy, (float)dz, margin, bb)) bb = sector_bits(dx, dy, dz);
                     sec |= bb;
@@ -866,7 +872,7 @@ __global__ void __launch_bounds__(256) k_filter_slots(int n, const int* __restri
         if (live && sub == 0) {
             cnt[i] = min(kept, maxn);
             if (kept > maxn) atomicAdd(trunc, (unsigned long long)(kept - maxn));
-            if (classify) cls[i] = classify_rule(stype[i], min(kept, maxn), sec, zi, l0);
+            if (classify) cls[i] = classify_rule(ti, min(kept, maxn), sec, zi, l0);
         }
     }
 }
