@@ -359,11 +359,11 @@ struct SegGrid {
 };
 
 // The decisions are safe when no component is within `margin` of zero and the largest is that far
-// above the other two.
+// above the other two (not so when two of them are beyond the FP32 range).
 __device__ __forceinline__ bool sector_bits_f32(float dx, float dy, float dz, float margin, unsigned& bits) {
     const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
     const float lo = fminf(ax, ay), hi = fmaxf(ax, ay), top = fmaxf(hi, az);
-    if (fminf(lo, az) <= margin || top - fmaxf(lo, fminf(hi, az)) <= margin) {
+    if (!(fminf(lo, az) > margin) || !(top - fmaxf(lo, fminf(hi, az)) > margin)) {
         bits = 0;
         return false;
     }
@@ -546,14 +546,16 @@ __global__ void __launch_bounds__(SEG_THREADS, 8) k_seg_pass(SegGrid G, const in
 // One warp per cell and 32 of its particles (the queries). The cell's candidates, the particles
 // of its 27 cells in the reference's order (9 rows of three cells, contiguous in the sorted
 // order), go into registers, one per lane and chunk of 32, as FP32 positions relative to the
-// cell's corner. The warp then takes the queries one by one: every lane tests its candidates
-// with packed FP32x2 arithmetic, the ballots of a chunk are the hits in order, the hits are
-// packed into shared memory and from there, a lane each, written to slots[k * maxn + p] for
-// p < maxn, with their sector bits for the classification. A query with a candidate in the
-// guard band of k_seg_pass (|d^2 - re^2| <= 2.1e-5 re^2; the FP32 distance^2 is within 1e-6 re^2
-// of the exact one) has its hits there decided exactly in FP64, so the kept lists are the
-// reference's bit for bit. Cells of more than SCAN_CH chunks take them in turns. Counting
-// continues past maxn for the truncation statistic. k_slots_compact then packs the slot rows
+// cell's corner in units of re (so that neither they nor their squares leave the FP32 range, and an
+// empty lane's marker lies far outside the radius, whatever re is). The warp then takes the queries
+// one by one: every lane tests its candidates with packed FP32x2 arithmetic, the ballots of a
+// chunk are the hits in order, the hits are packed into shared memory and from there, a lane each,
+// written to slots[k * maxn + p] for p < maxn, with their sector bits for the classification. A
+// query with a candidate in the guard band of k_seg_pass (|d^2 - re^2| <= 2.1e-5 re^2; the FP32
+// distance^2 is within 3e-6 re^2 of the exact one, out to 2^31 cells from the origin) has its hits
+// there decided exactly in FP64, so the kept lists are the reference's bit for bit. Cells of more
+// than SCAN_CH chunks take them in turns. Counting continues past maxn for the truncation
+// statistic. k_slots_compact then packs the slot rows
 // into the CSR once the kept counts are scanned.
 // What bounds it: the latency of a query's chain (ballots, packing, sector bits) at 16 warps per
 // SM; two queries at a time hide half of it (one at a time took 518 us at 1M). It took the place
@@ -566,9 +568,15 @@ __global__ void __launch_bounds__(SEG_THREADS, 8) k_seg_pass(SegGrid G, const in
 constexpr int SCAN_CH = 10;     // chunks of 32 candidates in registers (a cell of side 2.1 has 250 candidates)
 constexpr int SCAN_WARPS = 4;   // per block
 
+// The scan's FP32 limits on d^2 / re^2: above hi no neighbor, below lo one, between them the exact
+// test; queries with a candidate within `band` of 1 look.
+struct ScanBand {
+    float lo, hi, band;
+};
+
 // Items of the scan (cell x, y, z and first query), in any order (an item's outputs are addressed by its
 // own particles): items[0].x is their number, items[0].y how many the scan has drawn. rel: each particle's position relative to its
-// cell's corner, and the cell's x index.
+// cell's corner in units of re, and the cell's x index.
 __global__ void k_scan_prep(GridView g, int3 g0, double re, long long ncells, int n, const int* __restrict__ scell,
                             const double* __restrict__ sx, const double* __restrict__ sy,
                             const double* __restrict__ sz, int4* __restrict__ items, float4* __restrict__ rel) {
@@ -594,23 +602,21 @@ __global__ void k_scan_prep(GridView g, int3 g0, double re, long long ncells, in
     }
     if (t < n) {
         const int lin = scell[t], cx = lin % g.nx, u = lin / g.nx, cy = u % g.ny, cz = u / g.ny;
-        rel[t] = make_float4((float)(sx[t] - (g0.x + cx) * re), (float)(sy[t] - (g0.y + cy) * re),
-                             (float)(sz[t] - (g0.z + cz) * re), __int_as_float(cx));
+        rel[t] = make_float4((float)((sx[t] - (g0.x + cx) * re) / re), (float)((sy[t] - (g0.y + cy) * re) / re),
+                             (float)((sz[t] - (g0.z + cz) * re) / re), __int_as_float(cx));
     }
 }
 
 __global__ void __launch_bounds__(32 * SCAN_WARPS, 4) k_cell_scan(
     GridView g, int n, int4* __restrict__ items, const float4* __restrict__ rel, const double* __restrict__ sx,
-    const double* __restrict__ sy, const double* __restrict__ sz, const uint8_t* __restrict__ stype, float re_f,
+    const double* __restrict__ sy, const double* __restrict__ sz, const uint8_t* __restrict__ stype, ScanBand lim,
     double re2, int maxn, double l0, int classify, int* __restrict__ cnt, unsigned long long* trunc_total,
     int* __restrict__ slots, uint8_t* __restrict__ cls) {
     __shared__ float4 packed[SCAN_WARPS][2 * 32 * SCAN_CH];  // two queries' hits: position and index
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     float4* hits = packed[warp];
-    const float re2f = (float)re2;
-    const float lo_th = re2f * (1.f - 2e-5f), hi_th = re2f * (1.f + 2e-5f), band = 2.1e-5f * re2f;
-    const float margin = 4e-6f * re_f;
+    constexpr float margin = 4e-6f;  // units of re, as lim
     const int nitems = items[0].x;
     // An item's number, cell, row ranges and candidates are four dependent loads: the first three
     // are made one to three items ahead. The first items go by the warp's number, the others are
@@ -684,16 +690,16 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS, 4) k_cell_scan(
                     if (j < total) {
                         const float4 p = rel[mm];
                         m[c] = mm;
-                        x[c] = p.x + (float)(__float_as_int(p.w) - cx) * re_f;
-                        y[c] = p.y + (float)(r % 3 - 1) * re_f;
-                        z[c] = p.z + (float)(r / 3 - 1) * re_f;
+                        x[c] = p.x + (float)(__float_as_int(p.w) - cx);
+                        y[c] = p.y + (float)(r % 3 - 1);
+                        z[c] = p.z + (float)(r / 3 - 1);
                     }
                 }
             }
             // two queries at a time, so that one's chain of ballot, packing and sector bits fills the
             // other's waits (an odd last query goes twice, the second time without results)
             for (int q = 0; q < nq; q += 2) {
-                float qx[2], qy[2], qz[2], near = re2f;
+                float qx[2], qy[2], qz[2], near = 1.f;
                 unsigned bal[2][SCAN_CH];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
@@ -714,14 +720,14 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS, 4) k_cell_scan(
                             float2 d2 = __fmul2_rn(dx, dx);
                             d2 = __ffma2_rn(dy, dy, d2);
                             d2 = __ffma2_rn(dz, dz, d2);
-                            const float2 o = __fadd2_rn(d2, make_float2(-re2f, -re2f));
+                            const float2 o = __fadd2_rn(d2, make_float2(-1.f, -1.f));
                             near = fminf(near, fminf(fabsf(o.x), fabsf(o.y)));
-                            bal[h][c] = __ballot_sync(0xffffffffu, d2.x <= hi_th && m[c] != qb + q + h);
-                            bal[h][c + 1] = __ballot_sync(0xffffffffu, d2.y <= hi_th && m[c + 1] != qb + q + h);
+                            bal[h][c] = __ballot_sync(0xffffffffu, d2.x <= lim.hi && m[c] != qb + q + h);
+                            bal[h][c + 1] = __ballot_sync(0xffffffffu, d2.y <= lim.hi && m[c + 1] != qb + q + h);
                         }
                     }
                 }
-                if (__any_sync(0xffffffffu, near <= band)) {
+                if (__any_sync(0xffffffffu, near <= lim.band)) {
 #pragma unroll 1
                     for (int h = 0; h < 2; ++h) {
                         const int kq = qb + min(q + h, nq - 1);
@@ -732,7 +738,7 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS, 4) k_cell_scan(
                             if (ok) {
                                 const float dx = x[c] - (h ? qx[1] : qx[0]), dy = y[c] - (h ? qy[1] : qy[0]),
                                             dz = z[c] - (h ? qz[1] : qz[0]);
-                                if (dx * dx + dy * dy + dz * dz >= lo_th)
+                                if (dx * dx + dy * dy + dz * dz >= lim.lo)
                                     ok = xnorm2(xsub(sx[m[c]], sx[kq]), xsub(sy[m[c]], sy[kq]),
                                                 xsub(sz[m[c]], sz[kq])) < re2;
                             }
@@ -1036,9 +1042,12 @@ static void launch_cell_scan(lsmps_ctx* ctx, int maxn, double l0, int classify, 
     const size_t n = ctx->n, most = std::min((size_t)ctx->ncells, n) + n / 32 + 1;
     const unsigned grid = (unsigned)std::min<size_t>((most + SCAN_WARPS - 1) / SCAN_WARPS, 148 * 4);
     if (again) LSMPS_CUDA(cudaMemsetAsync(&ctx->scan_items.get<int4>()->y, 0, sizeof(int), ctx->stream));
+    // where re^2 itself leaves the FP64 range every candidate (d^2 <= 12 re^2) is decided exactly
+    const bool in_range = ctx->re2 > 1e-290 && ctx->re2 < 1e290;
+    const ScanBand lim = in_range ? ScanBand{1.f - 2e-5f, 1.f + 2e-5f, 2.1e-5f} : ScanBand{0.f, 100.f, INFINITY};
     k_cell_scan<<<grid, 32 * SCAN_WARPS, 0, ctx->stream>>>(
         grid_view(ctx), (int)n, ctx->scan_items.get<int4>(), ctx->scan_rel.get<float4>(), ctx->sx.get<double>(),
-        ctx->sy.get<double>(), ctx->sz.get<double>(), ctx->stype.get<uint8_t>(), (float)ctx->re, ctx->re2, maxn, l0,
+        ctx->sy.get<double>(), ctx->sz.get<double>(), ctx->stype.get<uint8_t>(), lim, ctx->re2, maxn, l0,
         classify, cnt, trunc, slots, cls);
     LSMPS_CHECK_LAUNCH();
 }
