@@ -102,6 +102,13 @@ int lsmps_set_autotune(lsmps_ctx* ctx, int mode);
  * Writes at most cap bytes (NUL-terminated) to buf; *needed gets the full size + 1. */
 int lsmps_autotune_report(lsmps_ctx* ctx, char* buf, size_t cap, size_t* needed);
 
+/* Bound on the waits inside a kernel: the blocks of a one-launch solve (FP64, JACOBI, MIXED, LEARNED)
+ * meet at barriers, and a block that has polled one `polls` times ends the solve with
+ * LSMPS_ERR_TIMEOUT (the context stays usable). 0 lets every wait give up at once; the default is
+ * about ten seconds. No reference counterpart. */
+#define LSMPS_WAIT_DEFAULT (1 << 24)
+int lsmps_set_wait_limit(lsmps_ctx* ctx, int polls);
+
 /* ---- particles -------------------------------------------------------------------- */
 /* xyz: n x 3 doubles (x, y, z interleaved, as the reference's Particle::r); type: n
  * class bytes (only Wall is read by classification, src/lsmps.cpp:27). Host memory. */

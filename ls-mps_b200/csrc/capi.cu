@@ -298,6 +298,13 @@ int lsmps_set_autotune(lsmps_ctx* ctx, int mode) {
     });
 }
 
+int lsmps_set_wait_limit(lsmps_ctx* ctx, int polls) {
+    return guarded(ctx, [&] {
+        LSMPS_REQUIRE(polls >= 0, LSMPS_ERR_ARG, "the wait limit must not be negative");
+        ctx->wait_limit = polls;
+    });
+}
+
 int lsmps_autotune_report(lsmps_ctx* ctx, char* buf, size_t cap, size_t* needed) {
     return guarded(ctx, [&] {
         const std::string r = autotune_report(ctx);

@@ -67,6 +67,7 @@ struct lsmps_ctx {
     unsigned timing_pending = 0;
 
     lsmps_gpu::DevBuf dflags;      // int device error flags
+    int wait_limit = LSMPS_WAIT_DEFAULT;  // polls of a grid barrier before it gives up
     lsmps_gpu::DevBuf scratch;     // general reduction scratch
     lsmps_gpu::DevBuf scan_tmp;    // block sums of scans
     lsmps_gpu::DevBuf host_dummy;

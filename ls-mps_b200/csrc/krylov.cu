@@ -13,8 +13,8 @@
 // last-block sum in each, host-launched, an iteration took 35.0 us at 6,000 unknowns (17.5 now),
 // 52 us at 181k (37.9) and 117 us at 911k (102).
 //
-// Waits are bounded: a block that polls a barrier longer than SPIN_LIMIT times raises
-// DFLAG_TIMEOUT and ends, and so does every block after it.
+// Waits are bounded: a block that polls a barrier more often than the context's wait limit raises
+// DFLAG_TIMEOUT and ends, and so does every block that waits for it.
 #include <algorithm>
 #include <cmath>
 
@@ -29,7 +29,6 @@ namespace {
 constexpr int KT = 1024;             // threads per block, one block per SM
 constexpr int KW = KT / 32;
 constexpr int KMAXB = 256;           // blocks of a launch at most
-constexpr int SPIN_LIMIT = 1 << 24;  // polls of a barrier (seconds)
 
 // ---- grid barrier and sums ----------------------------------------------------------------
 struct Shared {
@@ -48,6 +47,7 @@ struct Comm {
     double* part;   // two copies of (2 x KMAXB) partial sums
     unsigned* ctr;  // arrivals since the launch
     int* dflag;
+    int limit;  // polls of a barrier; 0: every wait gives up
     unsigned epoch = 0;
     // (warp index shuffled so that the compiler knows it to be the same in all lanes)
     int warp, lane;
@@ -61,8 +61,8 @@ struct Comm {
         int polls = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
-        } while ((int)(v - target) < 0 && ++polls < SPIN_LIMIT);
-        if (polls >= SPIN_LIMIT) {
+        } while ((int)(v - target) < 0 && ++polls < limit);
+        if (polls >= limit) {
             atomicOr(dflag, DFLAG_TIMEOUT);
             sh.dead = 1;
             sh.done = 5;
@@ -458,6 +458,7 @@ Comm make_comm(lsmps_ctx* ctx, KrylovResult** out) {
     c.part = red;
     c.ctr = reinterpret_cast<unsigned*>(red + 4 * KMAXB);
     c.dflag = ctx->dflags.get<int>();
+    c.limit = ctx->wait_limit;
     return c;
 }
 

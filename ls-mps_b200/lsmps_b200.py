@@ -205,6 +205,7 @@ SIGNATURES = {
     "lsmps_download_pressure_particles": (C.c_int, [_vp, _vp, C.c_size_t, C.c_double]),
     "lsmps_download_pressure_particles_device": (C.c_int, [_vp, _vp, C.c_size_t, C.c_double]),
     "lsmps_set_autotune": (C.c_int, [_vp, C.c_int]),
+    "lsmps_set_wait_limit": (C.c_int, [_vp, C.c_int]),
     "lsmps_autotune_report": (C.c_int, [_vp, C.c_char_p, C.c_size_t, C.POINTER(C.c_size_t)]),
     "lsmps_mpnn_param_count": (C.c_size_t, []),
     "lsmps_mpnn_init": (C.c_int, [_vp, C.c_uint32]),
@@ -317,6 +318,10 @@ class Context:
     def set_autotune(self, mode):
         """0 off (fixed default launch shapes), 1 on, 2 on and forget earlier choices."""
         self._check(self.L.lsmps_set_autotune(self.h, mode))
+
+    def set_wait_limit(self, polls=1 << 24):
+        """Polls of a barrier inside a one-launch solve before it ends with ERR_TIMEOUT."""
+        self._check(self.L.lsmps_set_wait_limit(self.h, polls))
 
     def autotune_report(self):
         """[(key, shape, ms, is_best)] of every candidate the autotuner timed on this context."""
