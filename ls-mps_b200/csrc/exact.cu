@@ -300,6 +300,7 @@ void solve_exact(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_stats* ps
         launch_pdl(k_x_dots, n, SEQ_THREADS, SEQ_SMEM, s, prod, U + 1, U, st, op, o->tol, max_iter);
     };
     ev_record(ctx, 10);
+    ctx->have_solution = false;  // until the solve has succeeded: x is overwritten from here on
     k_x_start<<<vecs, 256, 0, s>>>(A, b, x, r, r0, p[0], v[0]);
     LSMPS_CHECK_LAUNCH();
     dots(1, OP_START);

@@ -1044,6 +1044,7 @@ static void solve_fast64(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_s
     const KrylovVecs V = krylov_vecs(ctx);
     const Sell<double> A = jacobi ? sell_scaled64(ctx) : sell_a64(ctx);
     const double* dinv = ctx->A_dinv.get<double>();
+    ctx->have_solution = false;  // until the solve has succeeded: x is overwritten from here on
     if (warm && jacobi) {  // the iteration works on y = D x
         k_scale_by_diag<<<1184, 256, 0, ctx->stream>>>(U, V.x, dinv);
         LSMPS_CHECK_LAUNCH();
@@ -1090,6 +1091,7 @@ static void solve_mixed_f32(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_pp
     Sell<double> A = sell_a64(ctx);
     Sell<float> Af = sell_scaled32(ctx);
     set_scalar_caps(E, 0, 0);  // zero the reduction tickets
+    ctx->have_solution = false;  // until the solve has succeeded: x is overwritten from here on
     if (!warm) LSMPS_CUDA(cudaMemsetAsync(x, 0, U * sizeof(double), s));
     auto true_residual = [&]() {
         residual64(E, A, ctx->A_b.get<double>(), x, r64, scal);
@@ -1262,6 +1264,7 @@ static bool solve_mixed(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_st
     if (mg) {
         if (overlap) {
             side_stream_fork(ctx);
+            ctx->have_solution = false;  // as below
             net_guess();
             mg_setup_on_side(ctx);
         } else {
@@ -1283,6 +1286,7 @@ static bool solve_mixed(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_st
     ko.use_nn = use_nn;
     ko.dinv = dinv;
     ko.xe = ctx->A_xexact.get<double>();
+    ctx->have_solution = false;  // until the solve has succeeded: x is overwritten from here on
     if (warm) {  // the iteration works on y = D x
         k_scale_by_diag<<<1184, 256, 0, s>>>(U, V.x, dinv);
         LSMPS_CHECK_LAUNCH();

@@ -29,3 +29,28 @@ def test_wait_runs_out(built, n, solver):
         assert np.array_equal(ctx.pressure(n), x)
         with pytest.raises(lib.LsmpsError):
             ctx.set_wait_limit(-1)
+
+
+@pytest.mark.parametrize("solver", ["fp64", "jacobi", "mixed"])
+def test_no_solution_after_a_failed_solve(built, solver):
+    """what a failed solve leaves is a partial (column-scaled) iterate: it is neither handed out as a
+    solution nor continued by a warm start"""
+    n = 8191
+    row, col, val, b = system(n, 50, n)
+    with lib.Context(0) as ctx:
+        ctx.ppe_load_csr(row, col, val, b)
+        cold = ctx.ppe_solve(solver, 500, TOL)
+        x = ctx.pressure(n)
+        for warm in (False, True):
+            ctx.set_wait_limit(0)
+            with pytest.raises(lib.LsmpsError):
+                ctx.ppe_solve(solver, 500, TOL, warm_start=warm)
+            ctx.set_wait_limit()
+            with pytest.raises(lib.LsmpsError) as e:
+                ctx.pressure(n)
+            assert e.value.code == lib.ERR_STATE
+            again = ctx.ppe_solve(solver, 500, TOL, warm_start=True)  # nothing to start from
+            assert again.iterations == cold.iterations and np.array_equal(ctx.pressure(n), x)
+            with pytest.raises(lib.LsmpsError):  # refused before anything is written: the solution stays
+                ctx.ppe_solve(solver, 500, TOL, precond="multigrid")
+            assert np.array_equal(ctx.pressure(n), x)
