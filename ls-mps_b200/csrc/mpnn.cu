@@ -734,9 +734,9 @@ __global__ void __launch_bounds__(256) k_enc_bwd(GView G, const float* __restric
         gb[0] += g0;
         gb[1] += g1;
 #pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            gw[0][f] += g0 * x[f];
-            gw[1][f] += g1 * x[f];
+        for (int f = 0; f < NF; ++f) {  // (a masked gradient takes nothing from a non-finite feature)
+            if (g0 != 0.f) gw[0][f] += g0 * x[f];
+            if (g1 != 0.f) gw[1][f] += g1 * x[f];
         }
     }
 #pragma unroll
