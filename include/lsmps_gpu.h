@@ -109,6 +109,15 @@ int lsmps_autotune_report(lsmps_ctx* ctx, char* buf, size_t cap, size_t* needed)
 #define LSMPS_WAIT_DEFAULT (1 << 24)
 int lsmps_set_wait_limit(lsmps_ctx* ctx, int polls);
 
+/* SMs that this context's one-launch solves leave to the kernels of other contexts and streams
+ * (default 0). Such a solve keeps one block on every SM it takes, whose registers it fills, from
+ * its first iteration to its last, and starts when those SMs are free: above ~37,000 unknowns that is
+ * the whole GPU, and work of other contexts waits for the solve's end (5 to 20 ms at 1M particles).
+ * A program that runs several contexts at once gives them a few SMs (2: list builds of 20,000
+ * particles take 1.1 ms beside solves, and a MIXED iteration at 1M is 2 % slower). The sums'
+ * order goes by the blocks, so other values give other bits. No reference counterpart. */
+int lsmps_set_free_sms(lsmps_ctx* ctx, int sms);
+
 /* ---- particles -------------------------------------------------------------------- */
 /* xyz: n x 3 doubles (x, y, z interleaved, as the reference's Particle::r); type: n
  * class bytes (only Wall is read by classification, src/lsmps.cpp:27). Host memory. */

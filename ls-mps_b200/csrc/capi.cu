@@ -305,6 +305,15 @@ int lsmps_set_wait_limit(lsmps_ctx* ctx, int polls) {
     });
 }
 
+int lsmps_set_free_sms(lsmps_ctx* ctx, int sms) {
+    return guarded(ctx, [&] {
+        int all = 0;
+        LSMPS_CUDA(cudaDeviceGetAttribute(&all, cudaDevAttrMultiProcessorCount, ctx->device));
+        LSMPS_REQUIRE(sms >= 0 && sms < all, LSMPS_ERR_ARG, "a solve needs at least one SM");
+        ctx->free_sms = sms;
+    });
+}
+
 int lsmps_autotune_report(lsmps_ctx* ctx, char* buf, size_t cap, size_t* needed) {
     return guarded(ctx, [&] {
         const std::string r = autotune_report(ctx);

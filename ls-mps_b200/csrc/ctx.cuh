@@ -68,6 +68,7 @@ struct lsmps_ctx {
 
     lsmps_gpu::DevBuf dflags;      // int device error flags
     int wait_limit = LSMPS_WAIT_DEFAULT;  // polls of a grid barrier before it gives up
+    int free_sms = 0;  // SMs that one-launch solves leave to other contexts' kernels
     lsmps_gpu::DevBuf scratch;     // general reduction scratch
     lsmps_gpu::DevBuf scan_tmp;    // block sums of scans
     lsmps_gpu::DevBuf host_dummy;

@@ -441,11 +441,18 @@ __global__ void __launch_bounds__(KT, 1) k_row_product(const Sell<TM> A, const i
     }
 }
 
-// blocks of a launch: one per SM, fewer for small systems (at least eight slices each)
+// blocks of a launch: one per SM, less those the context leaves free; fewer for small systems (at
+// least eight slices each). A block fills its SM's register file for the whole solve
+// (milliseconds), so the kernels of other contexts and streams wait for its end unless SMs are left
+// to them: a 20,000-particle list build on another context took 35 ms beside FP64 solves at 1M and
+// 20 ms beside MIXED ones, 1.1 ms with two SMs left, 0.65 with four. Two cost 102.2 -> 104.4 us per
+// MIXED iteration at 911k unknowns (106.6 four) and other bits (the sums' order goes by blocks), so
+// none is the default.
 unsigned blocks(lsmps_ctx* ctx, long long nslices) {
     int sms = 0;
     LSMPS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    return (unsigned)std::max<long long>(1, std::min<long long>(std::min(sms, KMAXB), (nslices + 7) / 8));
+    const int most = std::max(1, std::min(sms - ctx->free_sms, KMAXB));
+    return (unsigned)std::max<long long>(1, std::min<long long>(most, (nslices + 7) / 8));
 }
 
 // zeroed barrier state behind the partial sums (all in ctx->red)

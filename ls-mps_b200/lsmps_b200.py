@@ -206,6 +206,7 @@ SIGNATURES = {
     "lsmps_download_pressure_particles_device": (C.c_int, [_vp, _vp, C.c_size_t, C.c_double]),
     "lsmps_set_autotune": (C.c_int, [_vp, C.c_int]),
     "lsmps_set_wait_limit": (C.c_int, [_vp, C.c_int]),
+    "lsmps_set_free_sms": (C.c_int, [_vp, C.c_int]),
     "lsmps_autotune_report": (C.c_int, [_vp, C.c_char_p, C.c_size_t, C.POINTER(C.c_size_t)]),
     "lsmps_mpnn_param_count": (C.c_size_t, []),
     "lsmps_mpnn_init": (C.c_int, [_vp, C.c_uint32]),
@@ -322,6 +323,10 @@ class Context:
     def set_wait_limit(self, polls=1 << 24):
         """Polls of a barrier inside a one-launch solve before it ends with ERR_TIMEOUT."""
         self._check(self.L.lsmps_set_wait_limit(self.h, polls))
+
+    def set_free_sms(self, sms=0):
+        """SMs that one-launch solves leave to other contexts' kernels (other values, other bits)."""
+        self._check(self.L.lsmps_set_free_sms(self.h, sms))
 
     def autotune_report(self):
         """[(key, shape, ms, is_best)] of every candidate the autotuner timed on this context."""
