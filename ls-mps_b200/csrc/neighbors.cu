@@ -574,37 +574,41 @@ struct ScanBand {
     float lo, hi, band;
 };
 
-// Items of the scan (cell x, y, z and first query), in any order (an item's outputs are addressed by its
-// own particles): items[0].x is their number, items[0].y how many the scan has drawn. rel: each particle's position relative to its
-// cell's corner in units of re, and the cell's x index.
-__global__ void k_scan_prep(GridView g, int3 g0, double re, long long ncells, int n, const int* __restrict__ scell,
+// Items of the scan (cell x, y, z and first query), in any order (an item's outputs are addressed by
+// its own particles): every 32nd particle of a cell makes one. items[0].x is their number,
+// items[0].y how many the scan has drawn. rel: each particle's position relative to its cell's
+// corner in units of re, and the cell's x index. (One thread per particle: with one per cell of the
+// dense grid a build of 100k particles over 512M cells took 7.4 ms, now 5.9. One addition to the
+// count per block: per warp it cost a 1M build 12 us.)
+__global__ void __launch_bounds__(256) k_scan_prep(GridView g, int3 g0, double re, int n, const int* __restrict__ scell,
                             const double* __restrict__ sx, const double* __restrict__ sy,
                             const double* __restrict__ sz, int4* __restrict__ items, float4* __restrict__ rel) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    int q0 = 0, blocks = 0;
-    if (t < ncells) {
-        q0 = g.cell_start[t];
-        blocks = (g.cell_start[t + 1] - q0 + 31) >> 5;
-    }
-    const int lane = threadIdx.x & 31;
-    int sum = blocks;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, sum, o);
-        if (lane >= o) sum += v;
-    }
-    int base = 0;
-    if (lane == 31 && sum) base = atomicAdd(&items[0].x, sum);
-    base = __shfl_sync(0xffffffffu, base, 31) + sum - blocks + 1;
-    if (blocks) {
-        const int u = (int)t / g.nx;
-        for (int b = 0; b < blocks; ++b)
-            items[base + b] = make_int4((int)t % g.nx, u % g.ny, u / g.ny, q0 + 32 * b);
-    }
+    int cx = 0, cy = 0, cz = 0;
+    bool first = false;
     if (t < n) {
-        const int lin = scell[t], cx = lin % g.nx, u = lin / g.nx, cy = u % g.ny, cz = u / g.ny;
+        const int lin = scell[t], u = lin / g.nx;
+        cx = lin % g.nx, cy = u % g.ny, cz = u / g.ny;
         rel[t] = make_float4((float)((sx[t] - (g0.x + cx) * re) / re), (float)((sy[t] - (g0.y + cy) * re) / re),
                              (float)((sz[t] - (g0.z + cz) * re) / re), __int_as_float(cx));
+        first = (((int)t - g.cell_start[lin]) & 31) == 0;
     }
+    __shared__ int before[9];  // items of the block's warps in front, then the block's first place
+    const unsigned m = __ballot_sync(0xffffffffu, first);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) before[warp] = __popc(m);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int sum = 0;
+        for (int w = 0; w < 8; ++w) {
+            const int c = before[w];
+            before[w] = sum;
+            sum += c;
+        }
+        before[8] = sum ? atomicAdd(&items[0].x, sum) + 1 : 0;
+    }
+    __syncthreads();
+    if (first) items[before[8] + before[warp] + __popc(m & ((1u << lane) - 1u))] = make_int4(cx, cy, cz, (int)t);
 }
 
 __global__ void __launch_bounds__(32 * SCAN_WARPS, 4) k_cell_scan(
@@ -1031,9 +1035,9 @@ static void scan_prep(lsmps_ctx* ctx) {
     int4* items = ctx->scan_items.ensure<int4>(most + 1);
     float4* rel = ctx->scan_rel.ensure<float4>(n);
     LSMPS_CUDA(cudaMemsetAsync(items, 0, sizeof(int4), s));
-    k_scan_prep<<<blocks_for(std::max(n, (size_t)ctx->ncells), 256), 256, 0, s>>>(
-        grid_view(ctx), make_int3(ctx->gmin[0], ctx->gmin[1], ctx->gmin[2]), ctx->re, ctx->ncells, (int)n,
-        ctx->scell.get<int>(), ctx->sx.get<double>(), ctx->sy.get<double>(), ctx->sz.get<double>(), items, rel);
+    k_scan_prep<<<blocks_for(n, 256), 256, 0, s>>>(
+        grid_view(ctx), make_int3(ctx->gmin[0], ctx->gmin[1], ctx->gmin[2]), ctx->re, (int)n, ctx->scell.get<int>(),
+        ctx->sx.get<double>(), ctx->sy.get<double>(), ctx->sz.get<double>(), items, rel);
     LSMPS_CHECK_LAUNCH();
 }
 
