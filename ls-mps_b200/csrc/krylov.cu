@@ -416,7 +416,8 @@ __global__ void __launch_bounds__(KT, 1) k_bicgstab(const Sell<TM> A, const Sell
     }
 }
 
-// The row product of an iteration on its own (kernel bench): v = A p and the partials of r0.v
+// The row product of an iteration on its own, for the kernel bench (a solve forms it inside
+// k_bicgstab): v = A p and the partials of r0.v
 template <class TM, bool C16>
 __global__ void __launch_bounds__(KT, 1) k_row_product(const Sell<TM> A, const int* cut, const double* p, double* v,
                                                        const double* r0, double* part) {
@@ -441,20 +442,6 @@ __global__ void __launch_bounds__(KT, 1) k_row_product(const Sell<TM> A, const i
     }
 }
 
-// blocks of a launch: one per SM, less those the context leaves free; fewer for small systems (at
-// least eight slices each). A block fills its SM's register file for the whole solve
-// (milliseconds), so the kernels of other contexts and streams wait for its end unless SMs are left
-// to them: a 20,000-particle list build on another context took 35 ms beside FP64 solves at 1M and
-// 20 ms beside MIXED ones, 1.1 ms with two SMs left, 0.65 with four. Two cost 102.2 -> 104.4 us per
-// MIXED iteration at 911k unknowns (106.6 four) and other bits (the sums' order goes by blocks), so
-// none is the default.
-unsigned blocks(lsmps_ctx* ctx, long long nslices) {
-    int sms = 0;
-    LSMPS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    const int most = std::max(1, std::min(sms - ctx->free_sms, KMAXB));
-    return (unsigned)std::max<long long>(1, std::min<long long>(most, (nslices + 7) / 8));
-}
-
 // zeroed barrier state behind the partial sums (all in ctx->red)
 Comm make_comm(lsmps_ctx* ctx, KrylovResult** out) {
     double* red = ctx->red.ensure<double>(4 * KMAXB + 64);
@@ -473,12 +460,26 @@ template <class TM, bool MIXED, bool C16>
 void launch(lsmps_ctx* ctx, Sell<TM> A, Sell<double> As, KrylovVecs V, KrylovOpts o, Comm C, KrylovResult* out) {
     auto k = k_bicgstab<TM, MIXED, C16>;
     void* args[] = {&A, &As, &V, &o, &C, &out};
-    LSMPS_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k), dim3(blocks(ctx, A.nslices)), dim3(KT), args, 0,
+    LSMPS_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k), dim3(krylov_blocks(ctx, A.nslices)), dim3(KT), args, 0,
                                            ctx->stream));
     note_launches(1);
 }
 
 }  // namespace
+
+// blocks of a launch: one per SM, less those the context leaves free; fewer for small systems (at
+// least eight slices each). A block fills its SM's register file for the whole solve
+// (milliseconds), so the kernels of other contexts and streams wait for its end unless SMs are left
+// to them: a 20,000-particle list build on another context took 35 ms beside FP64 solves at 1M and
+// 20 ms beside MIXED ones, 1.1 ms with two SMs left, 0.65 with four. Two cost 102.2 -> 104.4 us per
+// MIXED iteration at 911k unknowns (106.6 four) and other bits (the sums' order goes by blocks), so
+// none is the default.
+unsigned krylov_blocks(lsmps_ctx* ctx, long long nslices) {
+    int sms = 0;
+    LSMPS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    const int most = std::max(1, std::min(sms - ctx->free_sms, KMAXB));
+    return (unsigned)std::max<long long>(1, std::min<long long>(most, (nslices + 7) / 8));
+}
 
 KrylovResult krylov_solve(lsmps_ctx* ctx, const Sell<float>* Af, const Sell<double>& A, const KrylovVecs& V,
                           const KrylovOpts& o) {
@@ -502,8 +503,9 @@ template <class TM>
 void krylov_row_product(lsmps_ctx* ctx, const Sell<TM>& A, const int* cut, const double* p, double* v,
                         const double* r0) {
     double* part = ctx->red.ensure<double>(4 * KMAXB + 64);
-    if (A.dcol) k_row_product<TM, true><<<SELL_CUTS, KT, 0, ctx->stream>>>(A, cut, p, v, r0, part);
-    else k_row_product<TM, false><<<SELL_CUTS, KT, 0, ctx->stream>>>(A, cut, p, v, r0, part);
+    const unsigned nb = krylov_blocks(ctx, A.nslices);
+    if (A.dcol) k_row_product<TM, true><<<nb, KT, 0, ctx->stream>>>(A, cut, p, v, r0, part);
+    else k_row_product<TM, false><<<nb, KT, 0, ctx->stream>>>(A, cut, p, v, r0, part);
     LSMPS_CHECK_LAUNCH();
 }
 template void krylov_row_product<float>(lsmps_ctx*, const Sell<float>&, const int*, const double*, double*, const double*);

@@ -37,7 +37,9 @@ struct KrylovResult {
 // waits for the result. Af: the FP32 copy the mixed solvers iterate with (null: iterate with A).
 KrylovResult krylov_solve(lsmps_ctx* ctx, const Sell<float>* Af, const Sell<double>& A, const KrylovVecs& V,
                           const KrylovOpts& o);
-// v = A p and the block partials of r0.v, as an iteration forms them (no wait); cut: sell_cuts.
+// The blocks of a solve of nslices slices.
+unsigned krylov_blocks(lsmps_ctx* ctx, long long nslices);
+// v = A p and the block partials of r0.v over a solve's blocks, whose first slices cut holds (no wait).
 template <class TM>
 void krylov_row_product(lsmps_ctx* ctx, const Sell<TM>& A, const int* cut, const double* p, double* v, const double* r0);
 

@@ -614,12 +614,10 @@ __global__ void __launch_bounds__(32 * SB_WARPS) k_sell_build(
     if (!ok) atomicOr(bad, 1);
 }
 
-// cut[b]: the first slice of block b of SELL_CUTS, so that the blocks hold about the same number
-// of stored entries
+// cut[b]: the first slice of a solve's block b
 template <class T>
-__global__ void k_sell_cuts(Sell<T> A, int* __restrict__ cut) {
-    const int b = threadIdx.x;
-    if (b <= SELL_CUTS) cut[b] = (int)sell_cut(A, b, SELL_CUTS);
+__global__ void k_sell_cuts(Sell<T> A, unsigned blocks, int* __restrict__ cut) {
+    for (unsigned b = threadIdx.x; b <= blocks; b += blockDim.x) cut[b] = (int)sell_cut(A, b, blocks);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -979,8 +977,9 @@ static void sell_raw(lsmps_ctx* ctx) {
 
 template <class T>
 static const int* sell_cuts(lsmps_ctx* ctx, const Sell<T>& A) {
-    int* cut = ctx->S_cut.ensure<int>(SELL_CUTS + 1);
-    k_sell_cuts<<<1, 256, 0, ctx->stream>>>(A, cut);
+    const unsigned blocks = krylov_blocks(ctx, A.nslices);
+    int* cut = ctx->S_cut.ensure<int>(blocks + 1);
+    k_sell_cuts<<<1, 256, 0, ctx->stream>>>(A, blocks, cut);
     LSMPS_CHECK_LAUNCH();
     return cut;
 }

@@ -41,8 +41,6 @@ struct Sell {
     const int* rbase = nullptr;
 };
 
-constexpr int SELL_CUTS = 148;  // parts of a SELL copy for kernels of one block per SM
-
 // The assembled system's SELL copy with FP64 values of A (built on first use).
 Sell<double> sell_a64_view(lsmps_ctx* ctx);
 // The SELL copy of A D^-1 with FP32 values (built with the structure).
