@@ -5,9 +5,9 @@
  * two helper streams of its own carry the prefetched uploads (ordered before the context
  * stream by lsmps_use_prefetched_particles) and, in a LEARNED solve with the multigrid from a
  * cold start, the hierarchy set-up beside the network (joined back to the context stream
- * within the solve). Calls on one context are not
- * thread-safe, separate contexts are independent. Every function returns an
- * lsmps_status; lsmps_last_error() gives the message of the last failure.
+ * within the solve). Calls on one context are not thread-safe, separate contexts are independent
+ * (but share the GPU: lsmps_set_free_sms). Every function returns an lsmps_status;
+ * lsmps_last_error() gives the message of the last failure.
  *
  * Each entry point replaces one internal function of the reference benchmark
  * (lilux618/LS-MPS src/lsmps.cpp, which has no FFI of its own: these are the

@@ -11,8 +11,9 @@
 //     factors, and independent dots (s.s, t.t, t.s; r.r, r0.r) run side by side in one launch;
 //   * p and s are formed where the row products gather them, so an iteration is six launches
 //     instead of 18: v = A p, its dot, t = A s, three dots, the x / r update, two dots.
-// Per iteration of the rain_injection case (U = 6,000, 464 iterations; B200): 930 us before,
-// 102 us now = 3.2 (v) + 35 (r0.v) + 3.4 (t) + 22 (s.s, t.t, t.s) + 2.3 (x, r) + 34 (r.r, r0.r).
+// Per iteration of the shipped rain_injection configuration (U = 6,000; iterations 40 to 140; B200):
+// 918 us before, 100 us now = 4.4 (v) + 34.7 (r0.v) + 3.3 (t) + 19.6 (s.s, t.t, t.s) + 2.2 (x, r) +
+// 35.8 (r.r, r0.r); 507 and 81 us at U = 2,888 (smoke).
 // What is left is the additions of r0.v and r0.r, whose running value leaves its binade at
 // every second element, one after another: 6,000 of them at 8.2 cycles each are 25 us.
 #include <algorithm>

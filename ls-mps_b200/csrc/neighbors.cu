@@ -555,14 +555,14 @@ __global__ void __launch_bounds__(SEG_THREADS, 8) k_seg_pass(SegGrid G, const in
 // distance^2 is within 3e-6 re^2 of the exact one, out to 2^31 cells from the origin) has its hits
 // there decided exactly in FP64, so the kept lists are the reference's bit for bit. Cells of more
 // than SCAN_CH chunks take them in turns. Counting continues past maxn for the truncation
-// statistic. k_slots_compact then packs the slot rows
-// into the CSR once the kept counts are scanned.
-// What bounds it: the latency of a query's chain (ballots, packing, sector bits) at 16 warps per
-// SM; two queries at a time hide half of it (one at a time took 518 us at 1M). It took the place
-// of a block per 12-cell segment with a thread per query, which was bound by shared memory (24
-// bytes per candidate pair and lane) and by the divergent walk over each thread's hits, with 23
-// (mixed set) to 39 % (rain) of its warps' lanes idle: 532 us for 1M particles of a mixed set (479 now), 172 us for
-// 200k of a rain set (110) and 890 for 1M at radius 2.3 (496). Five blocks per SM (102
+// statistic. k_slots_compact then packs the slot rows into the CSR once the kept counts are scanned.
+// What bounds it: issue slots (70 % busy) and the latency of a query's chain (ballots, packing,
+// sector bits) at 16 warps per SM; two queries at a time hide half of the latter (one at a time took
+// 518 us at 1M when two took 479). It took the place of a block per 12-cell segment with a thread
+// per query, which was bound by shared memory (24 bytes per candidate pair and lane) and by the
+// divergent walk over each thread's hits, with 23 (mixed set) to 39 % (rain) of its warps' lanes
+// idle: 532 us for 1M particles of a mixed set (470 now), 172 us for 200k of a rain set (107) and
+// 890 for 1M at radius 2.3 (490). Five blocks per SM (102
 // registers, spilled) took 499 us, three 565. The sector bits are left out where the rule does not
 // read them (walls, a third of a rain set: 513 -> 496 us).
 constexpr int SCAN_CH = 10;     // chunks of 32 candidates in registers (a cell of side 2.1 has 250 candidates)

@@ -118,9 +118,9 @@ __global__ void k_ppe_exact(size_t n, int variant, const double* __restrict__ sx
 // entries go, in order, to the row's slot range at nbr_row[k] + k (room for every neighbor
 // plus the diagonal); k_ppe_pack moves them into the CSR once the row lengths are scanned.
 // Writes cnt[u] (entries with the diagonal), p*[u], b[u], D^-1[u].
-// stats (u64): [0] neumann, [1] failed rows. Bound by instruction issue (67 %): with the terms
-// passed by shuffles and added in every lane 470 us at 911k unknowns (417 now) and 897 at the
-// 3M rain series (803). Capped at 64 registers (8 blocks of 128 threads per SM).
+// stats (u64): [0] neumann, [1] failed rows. Bound by L1 (77 % of its peak) and the gathers'
+// latency: with the terms passed by shuffles and added in every lane 470 us at 911k unknowns (417
+// now) and 897 at the 3M rain series (803). Capped at 64 registers (8 blocks of 128 threads per SM).
 constexpr int PPE_G = 8;
 __global__ void __launch_bounds__(128, 8) k_ppe_rows(PpeParams P, long long U, const int* __restrict__ sorted_of_u,
                                                   const int* __restrict__ ref_of_u, const int* __restrict__ uidx,

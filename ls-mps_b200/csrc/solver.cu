@@ -1225,8 +1225,8 @@ static void side_stream_fork(lsmps_ctx* ctx) {
 // exit_res: {|b - A D^-1 y|, |b|} of the returned iterate when the solve converged (the
 // convergence test's own FP64 residual), else {-1, -1}. Returns whether ps holds the error
 // against p*. The Jacobi solves run in krylov.cu's one launch; the multigrid's launch the
-// iteration's kernels from the host, 2 x 11 + 5 of them, each under programmatic dependent launch
-// (the same steps between the grid barriers of one launch measured 370-400 against 290 us per
+// iteration's kernels from the host (2 x 9 + 5 of them with four coarse levels), each under programmatic dependent launch
+// (the same steps between the grid barriers of one launch measured 370-400 against 303 us per
 // iteration at 1M: one block of 1,024 threads per SM hides less of the V-cycle's dependent
 // loads than the kernels' 2,048 threads, and its shared memory takes the L1 from the row products).
 static bool solve_mixed(lsmps_ctx* ctx, const lsmps_solver_opts* o, lsmps_ppe_stats* ps, bool learned,

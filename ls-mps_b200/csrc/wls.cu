@@ -470,9 +470,9 @@ __device__ void atomic_max_nonneg(double* addr, double v) {
 
 // The right-hand sides accumulate in the moments' neighbor pass (one pass over the neighbors;
 // measured 22 % faster at 1M particles than a second right-hand-side pass, for 2 more registers).
-// Bound by the FP64 pipe's latency at 12 warps per SM. At 1M particles one analytic field takes
+// Bound by the FP64 pipe (64 % busy) and its latency at 12 warps per SM. At 1M particles one analytic field takes
 // 307 us (454 before the neighbor loop loaded one neighbor ahead and blocks were one warp), three
-// caller fields (ARRAY) 524 us (774, and 386 more for the copy of the solutions to the caller's
+// caller fields (ARRAY) 524 us (874, and 386 more for the copy of the solutions to the caller's
 // order, where they are now written directly).
 // One warp per block, so a warp's registers are free for the next one as soon as it ends (rows
 // of uneven length): blocks of 64 and 128 threads took 5 and 17 % longer.

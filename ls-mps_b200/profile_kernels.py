@@ -42,7 +42,7 @@ def main():
     ap.add_argument("--particles", type=int, default=1_000_000)
     ap.add_argument("--case", default="mixed")
     ap.add_argument("--reps", type=int, default=3)
-    ap.add_argument("--solve", choices=["fp64", "jacobi", "mixed", "learned"], default=None,
+    ap.add_argument("--solve", choices=["reference", "fp64", "jacobi", "mixed", "learned"], default=None,
                     help="also run one PPE solve to relative residual 1e-10")
     ap.add_argument("--precond", choices=["jacobi", "multigrid"], default="jacobi")
     ap.add_argument("--use-graph", type=int, default=1,
